@@ -121,7 +121,11 @@ struct ProjGeom {
     float vi_hi;                // largest valid row coordinate: float(H - 1.1)
     float load_scale;
     int pitch;                  // elements per projection row (>= W)
-    long long view_stride;      // elements between consecutive projections (H * pitch)
+    long long view_stride;      // elements between consecutive projections
+    // a stack that holds only some detector rows starts at detector row row0 and has
+    // `rows` of them (0: all H); its base pointer is that of detector row 0, which
+    // it may not hold
+    int row0 = 0, rows = 0;
 };
 
 ProjGeom proj_geom(const ctb_detector& det, const ctb_grid& grid, int z_begin, int z_end, float load_scale);
@@ -133,6 +137,8 @@ ProjGeom proj_geom(const ctb_detector& det, const ctb_grid& grid, int z_begin, i
 // bound applies.
 void row_band(const ctb_detector& det, const ctb_grid& grid, int z_begin, int z_end, const double* heights_px,
               int n_views, int* r_lo, int* rows);
+// The same for a slab's geometry and height offsets within [hlo, hhi].
+void slab_row_band(const ProjGeom& g, double hlo, double hhi, int* r_lo, int* rows);
 
 // Backprojection of views [0, n) from `views` (device view table) into vol.
 // hmax bounds |height offset| (pixels) over the views. Dispatches to the
@@ -142,6 +148,7 @@ int bp_pick_zc(int slab_slices);
 struct BpConfig {
     int zc = 0;     // z voxels per thread (8, 16 or 32): the block tile's height
     int nbuf = 0;   // projection boxes staged per CTA (2, 3 or 4): views in flight
+    bool scratch = true;   // may take device memory from the stream's pool for the call
 };
 int backproject_launch(const void* proj, int store_type, const float4* views, int n_views,
                        const ProjGeom& g, double hmax, float* vol, int accumulate, cudaStream_t s,
@@ -153,6 +160,15 @@ int backproject_global_launch(const void* proj, int store_type, const float4* vi
 int backproject_tma_launch(const void* proj, int store_type, const float4* views, int n_views,
                            const ProjGeom& g, double hmax, float* vol, int accumulate, cudaStream_t s,
                            int zc = 16, int nbuf = 0);
+// Whether the TMA kernel takes this layout (16-byte base and strides), and
+// whether its boxes fit this geometry.
+bool backproject_tma_layout(const void* proj, int store_type, const ProjGeom& g);
+bool backproject_tma_fits(int store_type, const ProjGeom& g, double hmax, int zc, int nbuf);
+// Copy rows row0 .. row0 + rows - 1 of n views (row pitch src_pitch, views
+// src_stride apart, any alignment of the element type) to dst, dense with
+// row pitch dst_pitch (a multiple of 16 bytes, dst 16-byte aligned).
+int repack_rows_launch(const void* src, int store_type, int W, int src_pitch, long long src_stride, int row0,
+                       int rows, int n, void* dst, int dst_pitch, cudaStream_t s);
 
 // Persistent multi-scan backprojection: one launch takes (scan, tile) work
 // items from a device counter until every scan of the batch is done.

@@ -715,22 +715,27 @@ void Reconstructor::worker_progress(DeviceWork& w, double frac, const float* pre
 // Ct/CtVolume.cpp:1155-1320, for one device's part of the volume).
 void row_band(const ctb_detector& det, const ctb_grid& grid, int z_begin, int z_end, const double* heights_px,
               int n_views, int* r_lo, int* rows) {
-    const int H = det.height;
     *r_lo = 0;
-    *rows = H;
+    *rows = det.height;
     if (z_end <= z_begin) return;
-    const ProjGeom ga = proj_geom(det, grid, z_begin, z_end, 1.0f);
     double hlo = 0, hhi = 0;
     for (int i = 0; i < n_views && heights_px; ++i) {
         hlo = std::min(hlo, heights_px[i]);
         hhi = std::max(hhi, heights_px[i]);
     }
+    slab_row_band(proj_geom(det, grid, z_begin, z_end, 1.0f), hlo, hhi, r_lo, rows);
+}
+
+void slab_row_band(const ProjGeom& ga, double hlo, double hhi, int* r_lo, int* rows) {
+    const int H = ga.H;
+    *r_lo = 0;
+    *rows = H;
     const double R = std::sqrt(double(ga.r2)) + 2.0 * double(ga.vs), D = ga.D;
     if (!(R < 0.9 * D)) return;
     // row vi = H/2 - (zw + h) U with zw = (j - zPre) vs, U = D / (D - s), |s| <= R
     const double Umin = D / (D + R), Umax = D / (D - R);
     const double a = (0.0 - double(ga.zPre)) * ga.vs + hlo;
-    const double b = (double(z_end - z_begin) - 1.0 - double(ga.zPre)) * ga.vs + hhi;
+    const double b = (double(ga.Zs) - 1.0 - double(ga.zPre)) * ga.vs + hhi;
     const double vmin = std::min(a * Umin, a * Umax), vmax = std::max(b * Umin, b * Umax);
     const int lo = std::max(0, int(std::floor(std::max(-1.0e9, double(H) / 2.0 - vmax))) - 3);
     const int hi = std::min(H - 1, int(std::floor(std::min(1.0e9, double(H) / 2.0 - vmin))) + 4);

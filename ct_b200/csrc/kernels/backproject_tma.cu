@@ -370,7 +370,7 @@ __device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __res
                            (bx.ovf_every > 0 && vv % bx.ovf_every == 0);
                 mbar_expect_tx(&p.full[b], uint32_t(bx.BU) * bx.BV * sizeof(T));
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                tma_load_3d(buf + size_t(b) * buf_stride, map, uo, vo, vv, &p.full[b]);
+                tma_load_3d(buf + size_t(b) * buf_stride, map, uo, vo - g.row0, vv, &p.full[b]);
             }
             __syncwarp();
         }
@@ -668,14 +668,26 @@ template <> struct TmaType<__nv_bfloat16> {
     static constexpr CUtensorMapDataType v = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
 };
 
-// Tensor map over [n_views][H][W] projections with row pitch g.pitch; columns
-// W..pitch-1 and everything outside the detector read as zero.
+// the rows of `proj` (the pointer of detector row 0) that exist
+template <typename T>
+const T* first_row(const T* proj, const ProjGeom& g) {
+    return proj + (long long)g.row0 * g.pitch;
+}
+template <typename T>
+bool tma_layout(const T* proj, const ProjGeom& g) {
+    return (size_t(g.pitch) * sizeof(T)) % 16 == 0 && (size_t(g.view_stride) * sizeof(T)) % 16 == 0 &&
+           (reinterpret_cast<uintptr_t>(first_row(proj, g)) & 15) == 0;
+}
+
+// Tensor map over [n_views][rows][W] projections with row pitch g.pitch; columns
+// W..pitch-1 and everything outside the rows held read as zero.
 template <typename T>
 bool make_map(const T* proj, int n_views, const ProjGeom& g, const Box& bx, CUtensorMap* map) {
-    if ((size_t(g.pitch) * sizeof(T)) % 16 != 0 || (reinterpret_cast<uintptr_t>(proj) & 15) != 0) return false;
+    if (!tma_layout(proj, g)) return false;
     auto enc = encode_fn();
     if (!enc) return false;
-    const cuuint64_t dims[3] = {cuuint64_t(g.W), cuuint64_t(g.H), cuuint64_t(n_views)};
+    proj = first_row(proj, g);
+    const cuuint64_t dims[3] = {cuuint64_t(g.W), cuuint64_t(g.rows > 0 ? g.rows : g.H), cuuint64_t(n_views)};
     const cuuint64_t strides[2] = {cuuint64_t(g.pitch) * sizeof(T), cuuint64_t(g.view_stride) * sizeof(T)};
     const cuuint32_t box[3] = {cuuint32_t(bx.BU), cuuint32_t(bx.BV), 1};
     const cuuint32_t estr[3] = {1, 1, 1};
@@ -684,8 +696,20 @@ bool make_map(const T* proj, int n_views, const ProjGeom& g, const Box& bx, CUte
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+constexpr size_t kMaxRing = 200 * 1024;   // dynamic shared memory of the box buffers
+
 // three box buffers when three CTAs still fit an SM's shared memory, else two
 int choose_nbuf(size_t per_buf) { return (3 * (3 * per_buf + 1024) <= 227 * 1024) ? 3 : 2; }
+
+template <typename T>
+bool tma_fits_t(const ProjGeom& g, double hmax, int zc, int nbuf_req) {
+    Box bx;
+    if (!box_dims(g, zc, hmax, sizeof(T), &bx)) return false;
+    const size_t per_buf = size_t(bx.buf_elems) * sizeof(T);
+    const int nbuf = (nbuf_req >= 2 && nbuf_req <= 4) ? nbuf_req : choose_nbuf(per_buf);
+    return size_t(nbuf) * per_buf <= kMaxRing && (g.Y + kTY - 1) / kTY <= 65535 &&
+           (g.Zs + g.z_begin % zc + zc - 1) / zc <= 65535;
+}
 
 template <typename T, int ZC>
 int launch_t(const T* proj, const float4* views, int n_views, const ProjGeom& g, double hmax, float* vol,
@@ -697,7 +721,7 @@ int launch_t(const T* proj, const float4* views, int n_views, const ProjGeom& g,
     const size_t per_buf = size_t(bx.buf_elems) * sizeof(T);
     const int nbuf = (nbuf_req >= 2 && nbuf_req <= 4) ? nbuf_req : choose_nbuf(per_buf);
     const size_t smem = size_t(nbuf) * per_buf;
-    if (smem > 200 * 1024) return CTB_ERR_UNSUPPORTED;
+    if (smem > kMaxRing) return CTB_ERR_UNSUPPORTED;
     auto kern = nbuf == 4 ? bp_tma_kernel<T, ZC, 4> : nbuf == 3 ? bp_tma_kernel<T, ZC, 3> : bp_tma_kernel<T, ZC, 2>;
     if (const int st = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) return st;
     dim3 grid((g.X + kTX - 1) / kTX, (g.Y + kTY - 1) / kTY, (g.Zs + g.z_begin % ZC + ZC - 1) / ZC);
@@ -768,7 +792,7 @@ int batch_plan_t(const BpBatchScan* scans, int n, BpBatchPlan* plan, int nbuf_re
     const size_t per_buf = size_t(max_elems) * sizeof(T);
     plan->nbuf = (nbuf_req >= 2 && nbuf_req <= 4) ? nbuf_req : choose_nbuf(per_buf);
     plan->smem = size_t(plan->nbuf) * per_buf;
-    if (plan->smem > 200 * 1024) return CTB_ERR_UNSUPPORTED;
+    if (plan->smem > kMaxRing) return CTB_ERR_UNSUPPORTED;
     auto kern = plan->nbuf == 4 ? bp_batch_kernel<T, ZC, 4>
               : plan->nbuf == 3 ? bp_batch_kernel<T, ZC, 3> : bp_batch_kernel<T, ZC, 2>;
     if (const int st = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), plan->smem)) return st;
@@ -816,6 +840,14 @@ int backproject_tma_launch(const void* proj, int store_type, const float4* views
             return launch_zc<__nv_bfloat16>(proj, views, n_views, g, hmax, vol, accumulate, zc, s, nbuf);
     }
     return CTB_ERR_UNSUPPORTED;
+}
+
+bool backproject_tma_layout(const void* proj, int store_type, const ProjGeom& g) {
+    return store_type == CTB_FP32 ? tma_layout((const float*)proj, g) : tma_layout((const __half*)proj, g);
+}
+
+bool backproject_tma_fits(int store_type, const ProjGeom& g, double hmax, int zc, int nbuf) {
+    return store_type == CTB_FP32 ? tma_fits_t<float>(g, hmax, zc, nbuf) : tma_fits_t<__half>(g, hmax, zc, nbuf);
 }
 
 int bp_batch_plan(int store_type, int zc, const BpBatchScan* scans, int n, BpBatchPlan* plan, int nbuf) {

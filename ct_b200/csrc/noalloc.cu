@@ -156,5 +156,7 @@ extern "C" int ctb_backproject_noalloc(const void* filtered, int store_type, int
     st = view_table_build(d_ang, d_h, n_views, d_views, s);
     if (st != CTB_OK) return st;
     const ProjGeom g = proj_geom(*det, *grid, z_begin, z_end, load_scale);
-    return backproject_launch(filtered, store_type, d_views, n_views, g, hmax, vol, accumulate, s);
+    BpConfig cfg;
+    cfg.scratch = false;   // rows the TMA kernel cannot take are gathered, not copied
+    return backproject_launch(filtered, store_type, d_views, n_views, g, hmax, vol, accumulate, s, cfg);
 }
