@@ -17,7 +17,13 @@
 // [u0, u0 + BU) x [v0, v0 + BV) of view iv. Boxes that reach outside the
 // detector read zeros (TMA out-of-bounds fill) which no in-bounds voxel uses.
 // A view whose footprint would not fit the box (BU, BV are host-side bounds
-// with margins) is flagged and read through global memory instead.
+// with margins) is flagged and read through global memory instead; a view whose
+// footprint misses the detector is neither loaded nor added. Columns that cross
+// the detector's row bounds run the pair loop on the groups of eight slices that
+// hold a kept one, the others masked. Both matter where the volume is as tall as
+// the detector and the cone cuts its ends: 360 views of 256 x 192 into 256^3 of
+// one pixel 3.77 -> 3.26 ms (FP32), 720 of 1024^2 into 512^3 56.97 -> 56.01 ms,
+// 120 of 200 x 152 into 96^3 0.322 -> 0.240 ms, bit-identical sums.
 //
 // Every mbarrier wait is bounded; a CTA that gives up records the failure in a
 // device counter (read by ctb_device_status) and stops issuing work.
@@ -174,6 +180,46 @@ __device__ __forceinline__ void column_pairs(const T* col, const int BU_run, con
     }
 }
 
+// The same for eight slices of which only those with their bit of `in` set are
+// summed: fzo the first one's offset in its block of 32 slices. The floor by
+// adding the magic number rounded toward zero holds for rows down to -2^22 too,
+// and a slice's row as int() and subtraction give it is the same unless the row
+// line's rounding puts a kept slice below row 0 (v_inside): that one keeps row 0.
+template <typename T>
+__device__ __forceinline__ void column_pairs_masked(const T* col, const int BU, float fzo, float c0b, float mdv,
+                                                    float fu, float w, unsigned in, float* acc, BoxRows br) {
+    constexpr float kMagic = 12582912.0f;   // 1.5 * 2^23
+    const float2 fu2 = make_float2(fu, fu), w2 = make_float2(w, w);
+    const float2 m1 = make_float2(-1.0f, -1.0f), mg = make_float2(kMagic, kMagic);
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+        const float2 vi = make_float2(fmaf(fzo + float(j), mdv, c0b), fmaf(fzo + float(j + 1), mdv, c0b));
+        const bool ina = in >> j & 1u, inb = in >> (j + 1) & 1u;
+        float2 sm = __fadd2_rz(vi, mg);
+        if (ina) sm.x = fmaxf(sm.x, kMagic);
+        if (inb) sm.y = fmaxf(sm.y, kMagic);
+        const float2 nfl = __ffma2_rn(sm, m1, mg);   // -float(floor(vi))
+        const float2 fv = __fadd2_rn(vi, nfl);
+        int rowa = __float_as_int(sm.x) - 0x4B400000, rowb = __float_as_int(sm.y) - 0x4B400000;
+#ifdef CTB_BOUNDS_CHECK
+        if (!CTB_FETCH_OK(rowa - br.oy, br.BV - 1, 1)) rowa = br.oy;
+        if (!CTB_FETCH_OK(rowb - br.oy, br.BV - 1, 1)) rowb = br.oy;
+#endif
+        const T* ra = col + rowa * BU;
+        const T* rb = col + rowb * BU;
+        const float2 p00 = make_float2(sval(ra[0]), sval(rb[0]));
+        const float2 p10 = make_float2(sval(ra[BU]), sval(rb[BU]));
+        const float2 d0 = make_float2(sub_from(ra[1], p00.x), sub_from(rb[1], p00.y));
+        const float2 d1 = make_float2(sub_from(ra[BU + 1], p10.x), sub_from(rb[BU + 1], p10.y));
+        const float2 a = __ffma2_rn(fu2, d0, p00);
+        const float2 c = __ffma2_rn(fu2, d1, p10);
+        const float2 r = __ffma2_rn(fv, __ffma2_rn(a, m1, c), a);
+        const float2 s = __ffma2_rn(w2, r, make_float2(acc[j], acc[j + 1]));
+        if (ina) acc[j] = s.x;
+        if (inb) acc[j + 1] = s.y;
+    }
+}
+
 // column_pairs with the two most common row strides compiled in (box_dims
 // gives 128 bytes times k plus 32: 80 or 144 texels of 16 bits, 72 or 40 of
 // 32 bits for voxels of one to two detector pixels), any other at run time.
@@ -231,6 +277,10 @@ struct Box {
 constexpr int kConsumerWarps = kTX * kTY / 32;
 constexpr int kThreads = (kConsumerWarps + 1) * 32;
 
+// A view of a tile: its box, texels from global memory (a footprint larger than
+// the box), or nothing.
+enum { kBoxed = 0, kGlobal = 1, kOffDetector = 2 };
+
 // Pipeline state in shared memory. Barrier phases are tracked through a
 // running box sequence number, so one CTA can run many tiles (persistent
 // kernel) through the same barriers.
@@ -241,7 +291,7 @@ struct Pipe {
     int2 org[NBUF];         // box origin (column, row)
     float4 qv[NBUF];        // {sin, cos, h} of the view in each buffer
     int vv[NBUF];           // index of the view in each buffer
-    int ovf[NBUF];          // footprint larger than the box: read global memory
+    int mode[NBUF];         // how the view is read: kBoxed, kGlobal, kOffDetector
     int abort_flag;         // a bounded wait gave up
     long long item;         // persistent kernel: current work item
 };
@@ -366,11 +416,19 @@ __device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __res
                 p.org[b] = make_int2(uo, vo);
                 p.qv[b] = q;
                 p.vv[b] = vv;
-                p.ovf[b] = (int(floorf(umax)) + 3 - uo > bx.BU) || (int(floorf(vmax)) + 3 - vo > bx.BV) ||
-                           (bx.ovf_every > 0 && vv % bx.ovf_every == 0);
-                mbar_expect_tx(&p.full[b], uint32_t(bx.BU) * bx.BV * sizeof(T));
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                tma_load_3d(buf + size_t(b) * buf_stride, map, uo, vo - g.row0, vv, &p.full[b]);
+                // no voxel of the tile on the detector (u and v are extreme at its corners; half a
+                // sample covers their rounding): nothing to load or add for this view
+                const bool off = vmax < -0.5f || vmin > bx.vi_hi + 0.5f || umax < -0.5f || umin > float(g.W) - 0.5f;
+                const bool ovf = (int(floorf(umax)) + 3 - uo > bx.BU) || (int(floorf(vmax)) + 3 - vo > bx.BV) ||
+                                 (bx.ovf_every > 0 && vv % bx.ovf_every == 0);
+                p.mode[b] = off ? kOffDetector : ovf ? kGlobal : kBoxed;
+                if (off) {
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&p.full[b])) : "memory");
+                } else {
+                    mbar_expect_tx(&p.full[b], uint32_t(bx.BU) * bx.BV * sizeof(T));
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    tma_load_3d(buf + size_t(b) * buf_stride, map, uo, vo - g.row0, vv, &p.full[b]);
+                }
             }
             __syncwarp();
         }
@@ -394,7 +452,8 @@ __device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __res
             }
         }
         if (aborted(abort_flag)) break;
-        if (live) {
+        const int mode = p.mode[b];
+        if (live && mode != kOffDetector) {
             const float4 q = p.qv[b];
             float U, u;
             column_geom(xw, yw, q.x, q.y, g.D, g.uOff, &U, &u);
@@ -408,7 +467,7 @@ __device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __res
                 // row_at(rl, zt + j): slice j sits zoff + j < 32 slices into the block
                 auto row_j = [&](int j) { return fmaf(fzoff + float(j), rl.mdv, c0b); };
                 const float vf = row_j(0), vl = row_j(ZC - 1);
-                if (!p.ovf[b]) {
+                if (mode == kBoxed) {
                     const int2 o = p.org[b];
                     int cu = u0 - o.x;   // column of u0 in the box
 #ifdef CTB_BOUNDS_CHECK
@@ -423,23 +482,16 @@ __device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __res
                         column_pairs_any<T, ZC, IMM>(col, BU, zoff, zo, c0b, rl.mdv, fu, w, acc,
                                                      BoxRows{o.y, bx.BV});
                     } else {
+                        // a column that crosses the row bounds: eight slices at a time, those that hold
+                        // a slice inside (the others' texels are in the box too; zeros past the detector)
                         int ja, jb;
                         v_inside_run(z0, ZC, g.zPre, g.vs, q.z, U, g.lbV, g.ubV, &ja, &jb);
+                        const unsigned in = ja <= jb ? (0xffffffffu << ja) & (0xffffffffu >> (31 - jb)) : 0u;
 #pragma unroll
-                        for (int j = 0; j < ZC; ++j) {
-                            const float vi = row_j(j);
-                            if (j >= ja && j <= jb) {
-                                int v0 = int(vi);
-                                const float fv = __fsub_rn(vi, float(v0));
-#ifdef CTB_BOUNDS_CHECK
-                                if (!CTB_FETCH_OK(v0 - o.y, bx.BV - 1, 1)) v0 = o.y;
-#endif
-                                const T* r0 = col + v0 * BU;
-                                const float p00 = sval(r0[0]), p10 = sval(r0[BU]);
-                                const float a = fmaf(fu, sub_from(r0[1], p00), p00);
-                                const float c = fmaf(fu, sub_from(r0[BU + 1], p10), p10);
-                                acc[j] = fmaf(w, fmaf(fv, c - a, a), acc[j]);
-                            }
+                        for (int j0 = 0; j0 < ZC; j0 += 8) {
+                            if (in >> j0 & 0xffu)
+                                column_pairs_masked<T>(col, BU, fzoff + float(j0), c0b, rl.mdv, fu, w, in >> j0,
+                                                       acc + j0, BoxRows{o.y, bx.BV});
                         }
                     }
                 } else {
