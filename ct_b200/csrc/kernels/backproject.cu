@@ -203,15 +203,10 @@ ProjGeom proj_geom(const ctb_detector& det, const ctb_grid& grid, int z_begin, i
 // z voxels per thread of the shared-memory backprojector: 32 spreads each
 // column's per-view geometry over twice the voxels of 16 (8% faster on the
 // 128-slice slabs of a 1024^3 volume, with 3 instead of 4 CTAs per SM; 64
-// at 2 CTAs per SM was slower again) when the slab holds whole tiles of 32
-// with at most 1/8 padding; thinner slabs take 16, or 8 for 8 slices or fewer.
-int bp_pick_zc(int Zs) {
-    for (int zc : {32, 16}) {
-        const int padded = (Zs + zc - 1) / zc * zc;
-        if (Zs >= 2 * zc && (padded - Zs) * 8 <= padded) return zc;
-    }
-    return Zs <= 8 ? 8 : 16;
-}
+// at 2 CTAs per SM was slower again). The slices of a slab's last tile that lie
+// past it cost little (a tile skips them in groups of eight), so slabs take the
+// smallest tile that holds 32, 16 or 8 slices.
+int bp_pick_zc(int Zs) { return Zs > 16 ? 32 : Zs > 8 ? 16 : 8; }
 
 namespace {
 

@@ -180,19 +180,19 @@ __device__ __forceinline__ void column_pairs(const T* col, const int BU_run, con
     }
 }
 
-// The same for eight slices of which only those with their bit of `in` set are
+// The same for N slices of which only those with their bit of `in` set are
 // summed: fzo the first one's offset in its block of 32 slices. The floor by
 // adding the magic number rounded toward zero holds for rows down to -2^22 too,
 // and a slice's row as int() and subtraction give it is the same unless the row
 // line's rounding puts a kept slice below row 0 (v_inside): that one keeps row 0.
-template <typename T>
+template <typename T, int N>
 __device__ __forceinline__ void column_pairs_masked(const T* col, const int BU, float fzo, float c0b, float mdv,
                                                     float fu, float w, unsigned in, float* acc, BoxRows br) {
     constexpr float kMagic = 12582912.0f;   // 1.5 * 2^23
     const float2 fu2 = make_float2(fu, fu), w2 = make_float2(w, w);
     const float2 m1 = make_float2(-1.0f, -1.0f), mg = make_float2(kMagic, kMagic);
 #pragma unroll
-    for (int j = 0; j < 8; j += 2) {
+    for (int j = 0; j < N; j += 2) {
         const float2 vi = make_float2(fmaf(fzo + float(j), mdv, c0b), fmaf(fzo + float(j + 1), mdv, c0b));
         const bool ina = in >> j & 1u, inb = in >> (j + 1) & 1u;
         float2 sm = __fadd2_rz(vi, mg);
@@ -277,9 +277,11 @@ struct Box {
 constexpr int kConsumerWarps = kTX * kTY / 32;
 constexpr int kThreads = (kConsumerWarps + 1) * 32;
 
-// A view of a tile: its box, texels from global memory (a footprint larger than
-// the box), or nothing.
-enum { kBoxed = 0, kGlobal = 1, kOffDetector = 2 };
+// A view of a tile: its box, its box for the slices that lie in the slab (a slab's
+// first and last tiles), texels from global memory (a footprint larger than the
+// box), or nothing. (The producer tells the consumers: they have no register to
+// spare for what is the same in every view.)
+enum { kBoxed = 0, kBoxedPart = 1, kGlobal = 2, kOffDetector = 3 };
 
 // Pipeline state in shared memory. Barrier phases are tracked through a
 // running box sequence number, so one CTA can run many tiles (persistent
@@ -291,7 +293,7 @@ struct Pipe {
     int2 org[NBUF];         // box origin (column, row)
     float4 qv[NBUF];        // {sin, cos, h} of the view in each buffer
     int vv[NBUF];           // index of the view in each buffer
-    int mode[NBUF];         // how the view is read: kBoxed, kGlobal, kOffDetector
+    int mode[NBUF];         // how the view is read
     int abort_flag;         // a bounded wait gave up
     long long item;         // persistent kernel: current work item
 };
@@ -315,12 +317,18 @@ __device__ __forceinline__ bool aborted(const volatile int* f) { return *f != 0;
 // tiles that start later start further on, so the CTAs resident at one time
 // read the same few views and share them in L2 (2.3x less DRAM traffic on a
 // 1024^3 slab of 1440 views of 2048^2).
-template <typename T, int ZC, int NBUF, bool IMM>
-__device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __restrict__ proj,
+// PART: the slab's first or last tiles may reach past it (else every tile holds ZC
+// slices of the slab; a kernel of its own, without the test 1 % faster).
+// SPLIT: this CTA takes n_views views from view0 on (views and map are the whole
+// set's) and leaves its sums in shared memory (the box buffers, `buf`: slice j of
+// column t at [j * 256 + t]) instead of storing them. Returns false when the tile
+// lies outside the cylinder (nothing to add up).
+template <typename T, int ZC, int NBUF, bool IMM, bool PART, bool SPLIT>
+__device__ __forceinline__ bool tile_pass(const CUtensorMap* map, const T* __restrict__ proj,
                                           const float4* __restrict__ views, int n_views, const ProjGeom& g,
                                           const Box& bx, int buf_stride, float* __restrict__ vol, int accumulate,
                                           int tile_x, int tile_y, int tile_z, Pipe<NBUF>& p, T* buf,
-                                          unsigned& seq, int rot, int zshift) {
+                                          unsigned& seq, int rot, int zshift, int view0 = 0) {
     volatile int* abort_flag = &p.abort_flag;
     // Consumer warp w covers an 8 (x) x 4 (y) patch of columns: its lanes then
     // sample a compact patch of the box (a few rows x ~12 words), which keeps
@@ -347,11 +355,11 @@ __device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __res
         const float ay = world_coord(y0, g.yPre, g.vs), byw = world_coord(y1, g.yPre, g.vs);
         const float dx = fmaxf(0.0f, fmaxf(ax, -bxw)), dy = fmaxf(0.0f, fmaxf(ay, -byw));
         if (dx * dx + dy * dy > g.r2 * 1.0001f + 1.0f) {
-            if (!producer && !accumulate && x < g.X && y < g.Y) {
+            if (!producer && !accumulate && x < g.X && y < g.Y && (!SPLIT || view0 == 0)) {
                 float* out = vol + (long long)y * g.X + x;
                 for (int j = zf; j < zl; ++j) out[(long long)(z0 + j) * plane] = 0.0f;
             }
-            return;
+            return false;
         }
     }
     const float xw = world_coord(x, g.xPre, g.vs);
@@ -386,7 +394,7 @@ __device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __res
             // footprint of the whole ZC tile (voxels past the slab end are evaluated
             // too and dropped at the store): project the 4 (x, y) corners at both z ends
             float umin = 3.0e38f, umax = -3.0e38f, vmin = 3.0e38f, vmax = -3.0e38f;
-            const int vv = rot ? (iv + rot) % n_views : iv;
+            const int vv = (rot ? (iv + rot) % n_views : iv) + (SPLIT ? view0 : 0);
             const float4 q = __ldg(&views[vv]);
             if (lane < 4) {
                 const int cx = (lane & 1) ? x1 : x0;
@@ -421,7 +429,7 @@ __device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __res
                 const bool off = vmax < -0.5f || vmin > bx.vi_hi + 0.5f || umax < -0.5f || umin > float(g.W) - 0.5f;
                 const bool ovf = (int(floorf(umax)) + 3 - uo > bx.BU) || (int(floorf(vmax)) + 3 - vo > bx.BV) ||
                                  (bx.ovf_every > 0 && vv % bx.ovf_every == 0);
-                p.mode[b] = off ? kOffDetector : ovf ? kGlobal : kBoxed;
+                p.mode[b] = off ? kOffDetector : ovf ? kGlobal : !PART || (zf == 0 && zl == ZC) ? kBoxed : kBoxedPart;
                 if (off) {
                     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&p.full[b])) : "memory");
                 } else {
@@ -433,7 +441,7 @@ __device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __res
             __syncwarp();
         }
         seq += iv;  // boxes issued (all of them unless a wait gave up)
-        return;
+        return true;
     }
 
     // -------------------------------------------------------------- consumers
@@ -467,7 +475,7 @@ __device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __res
                 // row_at(rl, zt + j): slice j sits zoff + j < 32 slices into the block
                 auto row_j = [&](int j) { return fmaf(fzoff + float(j), rl.mdv, c0b); };
                 const float vf = row_j(0), vl = row_j(ZC - 1);
-                if (mode == kBoxed) {
+                if (mode == kBoxed || (PART && mode == kBoxedPart)) {
                     const int2 o = p.org[b];
                     int cu = u0 - o.x;   // column of u0 in the box
 #ifdef CTB_BOUNDS_CHECK
@@ -478,27 +486,34 @@ __device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __res
                     // strictly inside the row bounds (half-pixel margin): every voxel of the column passes
                     // the per-voxel membership test, so this loop and the checked one take the same
                     // decisions
-                    if (fminf(vf, vl) >= 0.5f && fmaxf(vf, vl) <= g.vi_hi - 0.5f) {
+                    const bool inside = fminf(vf, vl) >= 0.5f && fmaxf(vf, vl) <= g.vi_hi - 0.5f;
+                    if (inside && (!PART || mode == kBoxed)) {
                         column_pairs_any<T, ZC, IMM>(col, BU, zoff, zo, c0b, rl.mdv, fu, w, acc,
                                                      BoxRows{o.y, bx.BV});
                     } else {
-                        // a column that crosses the row bounds: eight slices at a time, those that hold
-                        // a slice inside (the others' texels are in the box too; zeros past the detector)
-                        int ja, jb;
-                        v_inside_run(z0, ZC, g.zPre, g.vs, q.z, U, g.lbV, g.ubV, &ja, &jb);
-                        const unsigned in = ja <= jb ? (0xffffffffu << ja) & (0xffffffffu >> (31 - jb)) : 0u;
+                        // a column that crosses the row bounds, or a tile the slab: a few slices at a
+                        // time, those groups that hold a slice to sum (the others' texels are in the box
+                        // too; zeros past the detector)
+                        // slices zf .. zl - 1 of the tile lie in the slab
+                        unsigned in = PART ? (0xffffffffu << zf) & (0xffffffffu >> (32 - zl)) : 0xffffffffu;
+                        if (!inside) {
+                            int ja, jb;
+                            v_inside_run(z0, ZC, g.zPre, g.vs, q.z, U, g.lbV, g.ubV, &ja, &jb);
+                            in &= ja <= jb ? (0xffffffffu << ja) & (0xffffffffu >> (31 - jb)) : 0u;
+                        }
+                        constexpr int kGroup = ZC == 8 ? 2 : 8;
 #pragma unroll
-                        for (int j0 = 0; j0 < ZC; j0 += 8) {
-                            if (in >> j0 & 0xffu)
-                                column_pairs_masked<T>(col, BU, fzoff + float(j0), c0b, rl.mdv, fu, w, in >> j0,
-                                                       acc + j0, BoxRows{o.y, bx.BV});
+                        for (int j0 = 0; j0 < ZC; j0 += kGroup) {
+                            if (in >> j0 & ((1u << kGroup) - 1))
+                                column_pairs_masked<T, kGroup>(col, BU, fzoff + float(j0), c0b, rl.mdv, fu, w, in >> j0,
+                                                               acc + j0, BoxRows{o.y, bx.BV});
                         }
                     }
                 } else {
                     // the view staged in this buffer (the tile's view order is rotated)
                     int gv = p.vv[b], gu = u0;
 #ifdef CTB_BOUNDS_CHECK
-                    if (!CTB_FETCH_OK(gv, n_views, 5)) gv = 0;
+                    if (!CTB_FETCH_OK(gv - (SPLIT ? view0 : 0), n_views, 5)) gv = SPLIT ? view0 : 0;
                     if (!CTB_FETCH_OK(gu, g.W - 1, 3)) gu = 0;
 #endif
                     const T* col = proj + (long long)gv * g.view_stride + gu;
@@ -527,7 +542,15 @@ __device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __res
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&p.empty[b])) : "memory");
     }
     seq += n_views;
-    if (aborted(abort_flag) || x >= g.X || y >= g.Y) return;
+    if constexpr (SPLIT) {
+        // every consumer warp is done with the boxes before the sums take their place
+        asm volatile("bar.sync 1, %0;" ::"n"(kConsumerWarps * 32) : "memory");
+        float* sums = reinterpret_cast<float*>(buf);
+#pragma unroll
+        for (int j = 0; j < ZC; ++j) sums[j * (kConsumerWarps * 32) + tid] = acc[j];
+        return true;
+    }
+    if (aborted(abort_flag) || x >= g.X || y >= g.Y) return true;
     // (slice z0 + j of column (x, y); z0 < 0 only for slices j < zf, which are not stored)
     float* out = vol + (long long)z0 * plane + (long long)y * g.X + x;
 #pragma unroll
@@ -537,6 +560,7 @@ __device__ __forceinline__ void tile_pass(const CUtensorMap* map, const T* __res
             *o = accumulate ? (*o + acc[j]) : acc[j];
         }
     }
+    return true;
 }
 
 // After an abort: bounded drain of the last NBUF issued boxes (those may still
@@ -551,7 +575,7 @@ __device__ void pipe_abort_drain(Pipe<NBUF>& p, unsigned seq) {
     }
 }
 
-template <typename T, int ZC, int NBUF>
+template <typename T, int ZC, int NBUF, bool PART>
 __global__ void __launch_bounds__(kThreads, ZC > 16 ? 3 : 4) bp_tma_kernel(const __grid_constant__ CUtensorMap map,
                                                           const T* __restrict__ proj,
                                                           const float4* __restrict__ views, int n_views,
@@ -566,8 +590,74 @@ __global__ void __launch_bounds__(kThreads, ZC > 16 ? 3 : 4) bp_tma_kernel(const
     // k / resident of a tile's time after the first, so it starts that far on
     const long long k = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * blockIdx.z);
     const int rot = int((k % resident) * n_views / resident);
-    tile_pass<T, ZC, NBUF, true>(&map, proj, views, n_views, g, bx, bx.buf_elems, vol, accumulate, blockIdx.x,
+    tile_pass<T, ZC, NBUF, true, PART, false>(&map, proj, views, n_views, g, bx, bx.buf_elems, vol, accumulate, blockIdx.x,
                            blockIdx.y, blockIdx.z, p, reinterpret_cast<T*>(smem_raw), seq, rot, g.z_begin % ZC);
+    __syncthreads();
+    if (threadIdx.x == kConsumerWarps * 32 && p.abort_flag) pipe_abort_drain(p, seq);
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The same tiles with the views split among the `splits` CTAs of a cluster, for
+// grids that leave SM slots idle: a CTA's eight consumer warps run at their own
+// latency (about nine cycles per instruction, alone on an SM or with two
+// others), so a grid below three CTAs per SM leaves that share of the chip
+// unused. Each CTA sums its run of the views, the cluster adds the sums up through
+// distributed shared memory in a fixed order, CTA r the slices of its r-th
+// part. 96^3 voxels from 120 views of 200 x 152 (108 tiles on 148 SMs) 0.240 -> 0.134
+// ms, 64^3 from 180 views 0.367 -> 0.076 ms.
+template <typename T, int ZC, int NBUF>
+__global__ void __launch_bounds__(kThreads, ZC > 16 ? 3 : 4) bp_split_kernel(const __grid_constant__ CUtensorMap map,
+                                                            const T* __restrict__ proj,
+                                                            const float4* __restrict__ views, int n_views,
+                                                            ProjGeom g, Box bx, float* __restrict__ vol,
+                                                            int accumulate, int resident, int splits) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    __shared__ __align__(16) Pipe<NBUF> p;
+    if (threadIdx.x == 0) pipe_init(p);
+    __syncthreads();
+    unsigned seq = 0;
+    const int rank = blockIdx.z % splits, tile_z = blockIdx.z / splits;   // cluster of 1 x 1 x splits
+    const int va = int((long long)n_views * rank / splits), vb = int((long long)n_views * (rank + 1) / splits);
+    const long long k = blockIdx.x + (long long)gridDim.x * (blockIdx.y + (long long)gridDim.y * tile_z);
+    const int rot = int((k % resident) * (vb - va) / resident);
+    const int zshift = g.z_begin % ZC;
+    const bool sums_left = tile_pass<T, ZC, NBUF, true, true, true>(&map, proj, views, vb - va, g, bx, bx.buf_elems, vol,
+                                                              accumulate, blockIdx.x, blockIdx.y, tile_z, p,
+                                                              reinterpret_cast<T*>(smem_raw), seq, rot, zshift, va);
+    if (sums_left) {   // the same for every CTA of the cluster (one tile)
+        cluster_barrier();
+        const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+        constexpr int kWX = kTX / 8;
+        const int x = blockIdx.x * kTX + (warp % kWX) * 8 + (lane & 7);
+        const int y = blockIdx.y * kTY + (warp / kWX) * 4 + (lane >> 3);
+        if (tid < kConsumerWarps * 32 && x < g.X && y < g.Y) {
+            const long long plane = (long long)g.X * g.Y;
+            const int z0 = tile_z * ZC - zshift;
+            const int ja = ZC * rank / splits, jb = ZC * (rank + 1) / splits;
+#pragma unroll 4
+            for (int j = ja; j < jb; ++j) {
+                float s = 0.0f;
+                for (int q = 0; q < splits; ++q) {
+                    uint32_t a;
+                    float v;
+                    asm("mapa.shared::cluster.u32 %0, %1, %2;"
+                        : "=r"(a)
+                        : "r"(smem_u32(smem_raw) + uint32_t(j * (kConsumerWarps * 32) + tid) * 4u), "r"(q));
+                    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+                    s += v;
+                }
+                const int z = z0 + j;
+                if (z >= 0 && z < g.Zs) {
+                    float* o = vol + z * plane + (long long)y * g.X + x;
+                    *o = accumulate ? (*o + s) : s;
+                }
+            }
+        }
+        cluster_barrier();   // the sums stay until every CTA has read them
+    }
     __syncthreads();
     if (threadIdx.x == kConsumerWarps * 32 && p.abort_flag) pipe_abort_drain(p, seq);
 }
@@ -628,7 +718,7 @@ __global__ void __launch_bounds__(kThreads, ZC > 16 ? 3 : 4) bp_batch_kernel(con
         if (p.item >= total || p.abort_flag) break;
         const ScanDesc& d = scans[s_scan];
         const int rot = int((p.item % gridDim.x) * d.n_views / gridDim.x);
-        tile_pass<T, ZC, NBUF, false>(&d.map, static_cast<const T*>(d.proj), d.views, d.n_views, sg, sbx, buf_stride,
+        tile_pass<T, ZC, NBUF, false, true, false>(&d.map, static_cast<const T*>(d.proj), d.views, d.n_views, sg, sbx, buf_stride,
                                d.vol, d.accumulate, s_tile[0], s_tile[1], s_tile[2], p,
                                reinterpret_cast<T*>(smem_raw), seq, rot, 0);
         __syncthreads();
@@ -753,6 +843,22 @@ constexpr size_t kMaxRing = 200 * 1024;   // dynamic shared memory of the box bu
 // three box buffers when three CTAs still fit an SM's shared memory, else two
 int choose_nbuf(size_t per_buf) { return (3 * (3 * per_buf + 1024) <= 227 * 1024) ? 3 : 2; }
 
+// CTAs that share a tile's views (1: no split): as few as give 2.7 CTAs per slot (4,
+// with 90 views or more for each), eight at most, four views each at least. Tiles differ (columns outside the
+// cylinder, views off the detector), so a grid of a few CTAs per slot ends
+// earlier than one of one or two; beyond that the adding up costs more. Times in
+// ms for 1 / 2 / 4 / 8 CTAs per tile: 64^3, 180 views (0.07 tiles per slot) 0.367 /
+// 0.185 / 0.101 / 0.076; 96^3, 120 (0.24) 0.240 / 0.170 / 0.153 / 0.134; 128^3, 360
+// (0.58) 0.792 / 0.730 / 0.615 / 0.623; 160^3, 360 (1.1) 1.44 / 1.15 / 1.14 / 1.18;
+// 200^3, 360 (2.7) 2.61 / 2.49 / 2.61 / 2.75; 224^3, 360 (3.1) 3.11 / 3.00 / 3.13;
+// 256^3, 360 (4.6) 3.25 / 3.27 / 3.52.
+int choose_splits(long long tiles, int n_views, int slots) {
+    int sp = 1;
+    if (n_views >= 180 && tiles < 4LL * slots) sp = 2;
+    while (sp < 8 && n_views >= 8 * sp && 10 * tiles * sp < 27LL * slots) sp *= 2;
+    return sp;
+}
+
 template <typename T>
 bool tma_fits_t(const ProjGeom& g, double hmax, int zc, int nbuf_req) {
     Box bx;
@@ -772,9 +878,15 @@ int launch_t(const T* proj, const float4* views, int n_views, const ProjGeom& g,
     if (!make_map(proj, n_views, g, bx, &map)) return CTB_ERR_UNSUPPORTED;
     const size_t per_buf = size_t(bx.buf_elems) * sizeof(T);
     const int nbuf = (nbuf_req >= 2 && nbuf_req <= 4) ? nbuf_req : choose_nbuf(per_buf);
-    const size_t smem = size_t(nbuf) * per_buf;
+    size_t smem = size_t(nbuf) * per_buf;
     if (smem > kMaxRing) return CTB_ERR_UNSUPPORTED;
-    auto kern = nbuf == 4 ? bp_tma_kernel<T, ZC, 4> : nbuf == 3 ? bp_tma_kernel<T, ZC, 3> : bp_tma_kernel<T, ZC, 2>;
+    const bool part = g.z_begin % ZC != 0 || g.Zs % ZC != 0;
+    auto kern = part ? (nbuf == 4   ? bp_tma_kernel<T, ZC, 4, true>
+                        : nbuf == 3 ? bp_tma_kernel<T, ZC, 3, true>
+                                    : bp_tma_kernel<T, ZC, 2, true>)
+                     : (nbuf == 4   ? bp_tma_kernel<T, ZC, 4, false>
+                        : nbuf == 3 ? bp_tma_kernel<T, ZC, 3, false>
+                                    : bp_tma_kernel<T, ZC, 2, false>);
     if (const int st = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) return st;
     dim3 grid((g.X + kTX - 1) / kTX, (g.Y + kTY - 1) / kTY, (g.Zs + g.z_begin % ZC + ZC - 1) / ZC);
     if (grid.y > 65535 || grid.z > 65535) return CTB_ERR_UNSUPPORTED;
@@ -782,7 +894,30 @@ int launch_t(const T* proj, const float4* views, int n_views, const ProjGeom& g,
     CTB_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem));
     CTB_CUDA_TRY(cudaGetDevice(&dev));
     CTB_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    kern<<<grid, kThreads, smem, s>>>(map, proj, views, n_views, g, bx, vol, accumulate, std::max(1, per_sm * sms));
+    const int slots = std::max(1, per_sm * sms);
+    const int splits = choose_splits((long long)grid.x * grid.y * grid.z, n_views, slots);
+    if (splits > 1 && (long long)grid.z * splits <= 65535) {
+        auto kern_s = nbuf == 4 ? bp_split_kernel<T, ZC, 4>
+                    : nbuf == 3 ? bp_split_kernel<T, ZC, 3> : bp_split_kernel<T, ZC, 2>;
+        smem = std::max(smem, sizeof(float) * ZC * kConsumerWarps * 32);   // the sums take the boxes' place
+        if (const int st = ensure_dynamic_smem(reinterpret_cast<const void*>(kern_s), smem)) return st;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = 1;
+        at.val.clusterDim.y = 1;
+        at.val.clusterDim.z = splits;
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = dim3(grid.x, grid.y, grid.z * splits);
+        lc.blockDim = dim3(kThreads);
+        lc.dynamicSmemBytes = smem;
+        lc.stream = s;
+        lc.attrs = &at;
+        lc.numAttrs = 1;
+        return cuda_status(cudaLaunchKernelEx(&lc, kern_s, map, proj, views, n_views, g, bx, vol, accumulate,
+                                              std::max(1, slots / splits), splits),
+                           "bp_split_kernel launch");
+    }
+    kern<<<grid, kThreads, smem, s>>>(map, proj, views, n_views, g, bx, vol, accumulate, slots);
     return cuda_status(cudaGetLastError(), "bp_tma_kernel launch");
 }
 
