@@ -54,14 +54,15 @@ constexpr int kMaxFftLen = 8192;
 
 struct FilterPlan {
     int W = 0, pad = 0, filter = -1, M = 0, logM = 0;
-    float2* tw = nullptr;   // exp(-2 pi i k / M), k < M   (FP64-built, stored FP32)
+    float2* tw = nullptr;   // exp(-2 pi i k / M), k < M, and reordered (FP64-built, stored FP32)
     float* K = nullptr;     // real kernel spectrum, M entries (includes scaling)
 };
 
 // Transform length for a detector width and padding mode.
 int filter_transform_length(int W, int pad);
 // Build the twiddle and kernel-spectrum tables on the device (FP64 kernels).
-// tw and K must hold M entries each. Stream-ordered.
+// tw must hold filter_twiddle_count(M) entries, K M entries. Stream-ordered.
+int filter_twiddle_count(int M);
 int filter_build_tables(int W, int pad, int filter, int M, float2* tw, float* K, cudaStream_t s);
 
 // Device tables of a (W, pad, filter) triple on the current device, built on

@@ -833,7 +833,7 @@ int Reconstructor::run_pipeline(DeviceWork& w, float* out, int order, int z_lo, 
         auto need = [&](int sl) {
             const size_t nb = std::min<size_t>(3, (Zw + sl - 1) / sl);
             return view_filt * V + 3 * view_raw * chunk + nb * plane * sl * 4 * (convert ? 2 : 1) + 64 * V +
-                   size_t(M) * 12;
+                   size_t(M) * 24;
         };
         size_t have = w.d_filtered.bytes + w.d_ring.bytes;
         for (int b = 0; b < 3; ++b) have += w.d_slab[b].bytes + w.d_conv[b].bytes;
@@ -849,7 +849,7 @@ int Reconstructor::run_pipeline(DeviceWork& w, float* out, int order, int z_lo, 
         (st = w.d_views.ensure(sizeof(float4) * V, "view table")) ||
         (st = w.d_angles.ensure(sizeof(double) * V, "angles")) ||
         (st = w.d_heights.ensure(sizeof(double) * V, "height offsets")) ||
-        (st = w.d_tw.ensure(sizeof(float2) * M, "twiddles")) || (st = w.d_K.ensure(sizeof(float) * M, "filter")))
+        (st = w.d_tw.ensure(sizeof(float2) * filter_twiddle_count(M), "twiddles")) || (st = w.d_K.ensure(sizeof(float) * M, "filter")))
         return fail(st, global_error());
     // Slab boundaries: slabs of `slab` slices, and a last one of 32 slices cut
     // from a full-height last slab, so that the download no backprojection

@@ -40,7 +40,7 @@ int filter_tables(int W, int pad, int filter, cudaStream_t s, FilterTables* out)
     while ((1 << t.logM) < t.M) ++t.logM;
     float2* tw = nullptr;
     float* K = nullptr;
-    CTB_CUDA_TRY(cudaMalloc(&tw, sizeof(float2) * t.M));
+    CTB_CUDA_TRY(cudaMalloc(&tw, sizeof(float2) * filter_twiddle_count(t.M)));
     CTB_CUDA_TRY(cudaMalloc(&K, sizeof(float) * t.M));
     const int st = filter_build_tables(W, pad, filter, t.M, tw, K, s);
     if (st != CTB_OK) return st;

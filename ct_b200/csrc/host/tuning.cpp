@@ -133,7 +133,7 @@ int Reconstructor::autotune_locked(ctb_tuning* out) {
         (st = d_views.ensure(sizeof(float4) * Vs, "tuning view table")) ||
         (st = d_ang.ensure(sizeof(double) * Vs, "tuning angles")) ||
         (st = d_h.ensure(sizeof(double) * Vs, "tuning heights")) ||
-        (st = d_tw.ensure(sizeof(float2) * M, "tuning twiddles")) ||
+        (st = d_tw.ensure(sizeof(float2) * filter_twiddle_count(M), "tuning twiddles")) ||
         (st = d_K.ensure(sizeof(float) * M, "tuning filter")))
         return fail(st, global_error());
     for (int i = 0; i < Vs; ++i)

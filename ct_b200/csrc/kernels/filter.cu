@@ -20,10 +20,11 @@
 // Because K is real and even, two detector rows are filtered at once as the
 // real and imaginary parts of one complex signal.
 //
-// Each group of M/8 threads owns one row pair in shared memory (M complex
-// floats); the FFT is a Stockham radix-4 (+ one radix-2) autosort transform
-// with two barriers per stage. Raw pixels are read once, filtered values are
-// written once: HBM traffic is the algorithmic minimum.
+// Lengths 256 ... 4096 run in registers (filter_rf_kernel below). Otherwise each
+// group of M/8 threads owns one row pair in shared memory (M complex floats)
+// and the FFT is a Stockham autosort transform with two barriers per stage. Raw
+// pixels are read once, filtered values are written once: HBM traffic is the
+// algorithmic minimum.
 
 #include <type_traits>
 #include <cuda_bf16.h>
@@ -42,6 +43,16 @@ __global__ void twiddle_kernel(float2* tw, int M) {
     double s, c;
     sincospi(-2.0 * double(k) / double(M), &s, &c);
     tw[k] = make_float2(float(c), float(s));
+}
+
+// The same factors in the order the register transforms read them (a warp's lanes
+// side by side; the plain table's stride of s factors took up to 30 wavefronts a
+// load): w_M^(ts) at [M + s L + t], s < 16, t < L = M / 16, and w_L^(t2 s2) at
+// [2 M + s2 L2 + t2], s2 < 16, t2 < L2 = L / 16.
+__global__ void twiddle_order_kernel(float2* tw, int M) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, L = M / 16, L2 = L / 16;
+    if (k < M) tw[M + k] = tw[(k / L) * (k % L)];
+    else if (k < M + L) tw[M + k] = tw[16 * ((k - M) / L2) * ((k - M) % L2)];
 }
 
 // Reference window, Ct/CtVolume.cpp:868-885: rl = float(n)/float(N) in float,
@@ -368,237 +379,367 @@ __global__ void __launch_bounds__(1024) filter_kernel(const InT* __restrict__ ra
 }
 
 // --------------------------------------- register four-step transform
-// For M = 16 L with L = 16 L2 (M = 512 ... 4096) a group of L threads owns one
-// row pair. Every thread keeps 16 complex values in registers and the
-// transform is three register passes joined by two shared-memory transposes:
-//   1. thread t:       16-point DFT over r of x[t + L r], times w_M^(t s)
+// For M = 16 L with L = 16 L2 (M = 256 ... 4096) a group of L threads owns four
+// detector rows: rows r0, r0+1 as the real and imaginary parts of one complex
+// signal, r0+2, r0+3 of another. Every thread keeps 16 values of both, the two
+// signals side by side in FP32x2 pairs (real parts in one pair, imaginary parts
+// in another): every operation of the transform is one FP32x2 instruction for
+// both, a multiplication by i costs nothing, and the twiddles, the kernel
+// spectrum and the weights' addresses serve both. Three register passes joined
+// by two shared-memory transposes:
+//   1. thread t:       16-point DFT over r of x[t + L r], times w_M^(ts)
 //   2. thread (s, t2): 16-point DFT over r of pass 1's values (t2 + L2 r, s),
 //                      times w_L^(t2 s2)
-//   3. thread (s, j):  for s2 = j + L2 q (q < 16 / L2) the L2-point DFT over t2,
+//   3. thread (s, j):  for s2 = j + L2 q (q < 16 / L2) the L2-point DFT over t2
+//                      (none for M = 256, L2 = 1),
 // which leaves X[s + 16 s2 + 256 k3] in registers (k3 < L2). The kernel
 // spectrum multiplies it there; the inverse runs the passes backwards with
 // conjugate factors and ends with thread t holding x[t + L r] again, so raw
 // rows are read and filtered rows written with the same coalesced pattern.
 // The exchange between passes 2 and 3 stays inside a warp. The paddings (L2
 // per 16-value row of the first transpose, 1 per s2 row and L2 per s block of
-// the second) keep every shared-memory access at two wavefronts per warp (one
-// per half-warp, the minimum for 8-byte elements). Three block barriers per
-// row pair; four where the second transpose reuses the first one's space so
-// that three CTAs fit an SM.
+// the second) keep every shared-memory access of 16 bytes per lane at the four
+// wavefronts a warp needs.
+//
+// HALF: W <= M / 2 (rows embedded in a longer transform): the upper eight of a
+// thread's sixteen columns are zeros before and unused after the transform, so
+// they are neither loaded nor computed in the outer passes.
+//
+// What bounds it: the FP32 pipe (an FP32x2 instruction takes two of its cycles;
+// per sample of a power-of-two row about 35 operations of the transforms and 19 of
+// -ln, the weight and the scales), 16 warps per SM and the L1 pipe together: 56 % of
+// the issue slots, 55 % of the L1 wavefronts. 54 instructions per sample; the
+// version before (one row pair per group, scalar operations, twiddles read at a
+// stride) took 84. u16 to FP16, 144 views of 2048^2: 2.11 -> 1.56 ms (1.5 TB/s); 360 of
+// 701 x 409 to FP32 (M = 2048): 1.21 -> 0.64; 360 of 256 x 192 to FP16: 0.104 ->
+// 0.042. Not faster: one code instance for both row pairs (a loop; registers
+// spill: 1.77 ms), five CTAs of 128 threads per SM (102 registers: 1.81).
 template <int M> struct RF {
     static constexpr int L = M / 16, L2 = L / 16, Q = 16 / L2;
-    static constexpr int SA = 16 * (L + L2);       // first transpose, float2 per group
-    static constexpr int SB = 16 * (L2 + 1) + L2;  // second transpose, float2 per s block
-    static constexpr int G = 256 / L;              // row pairs per CTA of 256 threads
-    static constexpr bool ALIAS = 3 * (size_t(G) * (SA + 16 * SB) * 8 + 1024) > 227 * 1024;
-    static constexpr int SG = ALIAS ? (SA > 16 * SB ? SA : 16 * SB) : SA + 16 * SB;  // float2 per group
-    static_assert(M >= 512 && M <= 4096 && (M & (M - 1)) == 0, "register transform lengths");
+    static constexpr int SA = 16 * (L + L2);       // first transpose, float4 per group
+    static constexpr int SB = 16 * (L2 + 1) + L2;  // second transpose, float4 per s block
+    static constexpr int T = L > 128 ? L : 128;    // threads per CTA: small ones, whose barriers stall little
+    static constexpr int G = T / L;                // groups (of four rows) per CTA
+    static constexpr int SG = L2 > 1 && 16 * SB > SA ? 16 * SB : SA;   // float4 per group, both in one place
+    static_assert(M >= 256 && M <= 4096 && (M & (M - 1)) == 0, "register transform lengths");
 };
 
-__device__ __forceinline__ float2 cmul_conj(float2 a, float2 b) {
-    return make_float2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
+// two complex numbers side by side: (re of A, re of B), (im of A, im of B)
+struct C2 {
+    float2 x, y;
+};
+
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
+__device__ __forceinline__ C2 add2(const C2& a, const C2& b) { return {add2(a.x, b.x), add2(a.y, b.y)}; }
+__device__ __forceinline__ C2 sub2(const C2& a, const C2& b) { return {sub2(a.x, b.x), sub2(a.y, b.y)}; }
+
+// a times w (CONJ: its conjugate)
+template <bool CONJ>
+__device__ __forceinline__ C2 mul2(const C2& a, float2 w) {
+    const float2 c = dup(w.x), s = dup(w.y), n = dup(-w.y);
+    return {__ffma2_rn(a.y, CONJ ? s : n, __fmul2_rn(a.x, c)), __ffma2_rn(a.x, CONJ ? n : s, __fmul2_rn(a.y, c))};
+}
+
+// 4-point DFT in place (INV: the inverse); HALF_IN: v2 and v3 are zero
+template <bool INV, bool HALF_IN = false>
+__device__ __forceinline__ void dft4(C2& v0, C2& v1, C2& v2, C2& v3) {
+    const C2 a0 = HALF_IN ? v0 : add2(v0, v2), a1 = HALF_IN ? v0 : sub2(v0, v2);
+    const C2 a2 = HALF_IN ? v1 : add2(v1, v3), d = HALF_IN ? v1 : sub2(v1, v3);
+    v0 = add2(a0, a2);
+    v2 = sub2(a0, a2);
+    // a1 + and - (-i d forward, i d inverse)
+    const C2 p = {add2(a1.x, d.y), sub2(a1.y, d.x)}, m = {sub2(a1.x, d.y), add2(a1.y, d.x)};
+    v1 = INV ? m : p;
+    v3 = INV ? p : m;
+}
+
+template <bool INV>
+__device__ __forceinline__ void dft8(C2* v) {
+    C2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
+    C2 o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
+    dft4<INV>(e0, e1, e2, e3);
+    dft4<INV>(o0, o1, o2, o3);
+    // w^1 = (1 -+ i)/sqrt2, w^2 = -+i, w^3 = (-1 -+ i)/sqrt2 (upper sign: forward)
+    const float2 h = dup(kSqrtHalf), nh = dup(-kSqrtHalf);
+    const C2 t1 = INV ? C2{__fmul2_rn(h, sub2(o1.x, o1.y)), __fmul2_rn(h, add2(o1.x, o1.y))}
+                      : C2{__fmul2_rn(h, add2(o1.x, o1.y)), __fmul2_rn(h, sub2(o1.y, o1.x))};
+    const C2 t3 = INV ? C2{__fmul2_rn(nh, add2(o3.x, o3.y)), __fmul2_rn(h, sub2(o3.x, o3.y))}
+                      : C2{__fmul2_rn(h, sub2(o3.y, o3.x)), __fmul2_rn(nh, add2(o3.x, o3.y))};
+    v[0] = add2(e0, o0);
+    v[4] = sub2(e0, o0);
+    v[1] = add2(e1, t1);
+    v[5] = sub2(e1, t1);
+    const C2 p = {add2(e2.x, o2.y), sub2(e2.y, o2.x)}, m = {sub2(e2.x, o2.y), add2(e2.y, o2.x)};
+    v[2] = INV ? m : p;
+    v[6] = INV ? p : m;
+    v[3] = add2(e3, t3);
+    v[7] = sub2(e3, t3);
 }
 
 // x times w16^m (forward: exp(-2 pi i m / 16); inverse: the conjugate)
 template <bool INV, int m>
-__device__ __forceinline__ float2 tw16(float2 x) {
+__device__ __forceinline__ C2 tw16(const C2& a) {
     constexpr float c1 = 0.92387953251128675613f, s1 = 0.38268343236508977173f;
     // cos and sin of 2 pi m / 16 for m = 0 ... 9 (m = n1 k2 <= 9)
     constexpr float cs[10] = {1.0f, c1, kSqrtHalf, s1, 0.0f, -s1, -kSqrtHalf, -c1, -1.0f, -c1};
     constexpr float sn[10] = {0.0f, s1, kSqrtHalf, c1, 1.0f, c1, kSqrtHalf, s1, 0.0f, -s1};
     static_assert(m >= 0 && m <= 9, "twiddle index");
-    if constexpr (m == 0) return x;
-    else if constexpr (m == 4) return rot90<INV>(x);
-    else {
-        const float c = cs[m], sv = sn[m];
-        return INV ? make_float2(x.x * c - x.y * sv, x.y * c + x.x * sv)
-                   : make_float2(x.x * c + x.y * sv, x.y * c - x.x * sv);
+    if constexpr (m == 0) return a;
+    else if constexpr (m == 4) {
+        const float2 m1 = dup(-1.0f);
+        return INV ? C2{__fmul2_rn(a.y, m1), a.x} : C2{a.y, __fmul2_rn(a.x, m1)};
+    } else {
+        return mul2<!INV>(a, make_float2(cs[m], sn[m]));
     }
-}
-
-template <bool INV, int n1>
-__device__ __forceinline__ void tw16_row(float2* a) {
-    a[1] = tw16<INV, n1 * 1>(a[1]);
-    a[2] = tw16<INV, n1 * 2>(a[2]);
-    a[3] = tw16<INV, n1 * 3>(a[3]);
 }
 
 // 16-point DFT in registers, natural order in and out: n = n1 + 4 n2,
 // k = 4 k1 + k2; 4-point DFTs over n2, twiddles w16^(n1 k2), 4-point DFTs over n1.
-template <bool INV>
-__device__ __forceinline__ void dft16(float2* v) {
-    float2 a[4][4];
+// HALF_IN: the inputs 8 .. 15 are zero; HALF_OUT: only the outputs 0 .. 7 are wanted.
+template <bool INV, bool HALF_IN = false, bool HALF_OUT = false>
+__device__ __forceinline__ void dft16(C2* v) {
+    C2 a[4][4];
 #pragma unroll
     for (int n1 = 0; n1 < 4; ++n1) {
-        a[n1][0] = v[n1]; a[n1][1] = v[n1 + 4]; a[n1][2] = v[n1 + 8]; a[n1][3] = v[n1 + 12];
-        dft4<INV>(a[n1][0], a[n1][1], a[n1][2], a[n1][3]);
+        a[n1][0] = v[n1]; a[n1][1] = v[n1 + 4];
+        if constexpr (!HALF_IN) {
+            a[n1][2] = v[n1 + 8]; a[n1][3] = v[n1 + 12];
+        }
+        dft4<INV, HALF_IN>(a[n1][0], a[n1][1], a[n1][2], a[n1][3]);
     }
-    tw16_row<INV, 1>(a[1]);
-    tw16_row<INV, 2>(a[2]);
-    tw16_row<INV, 3>(a[3]);
+    a[1][1] = tw16<INV, 1>(a[1][1]); a[1][2] = tw16<INV, 2>(a[1][2]); a[1][3] = tw16<INV, 3>(a[1][3]);
+    a[2][1] = tw16<INV, 2>(a[2][1]); a[2][2] = tw16<INV, 4>(a[2][2]); a[2][3] = tw16<INV, 6>(a[2][3]);
+    a[3][1] = tw16<INV, 3>(a[3][1]); a[3][2] = tw16<INV, 6>(a[3][2]); a[3][3] = tw16<INV, 9>(a[3][3]);
 #pragma unroll
     for (int k2 = 0; k2 < 4; ++k2) {
         dft4<INV>(a[0][k2], a[1][k2], a[2][k2], a[3][k2]);
 #pragma unroll
-        for (int k1 = 0; k1 < 4; ++k1) v[4 * k1 + k2] = a[k1][k2];
+        for (int k1 = 0; k1 < (HALF_OUT ? 2 : 4); ++k1) v[4 * k1 + k2] = a[k1][k2];   // (unwanted ones: dead code)
     }
 }
 
+// L2-point DFT
 template <int N, bool INV>
-__device__ __forceinline__ void dft_n(float2* v) {
-    if constexpr (N == 2) dft2<INV>(v);
-    else if constexpr (N == 4) dft4<INV>(v[0], v[1], v[2], v[3]);
-    else if constexpr (N == 8) dft8<INV>(v);
-    else dft16<INV>(v);
+__device__ __forceinline__ void dft_n(C2* v) {
+    if constexpr (N == 2) {
+        const C2 a = v[0], b = v[1];
+        v[0] = add2(a, b);
+        v[1] = sub2(a, b);
+    } else if constexpr (N == 4) {
+        dft4<INV>(v[0], v[1], v[2], v[3]);
+    } else if constexpr (N == 8) {
+        dft8<INV>(v);
+    } else if constexpr (N == 16) {
+        dft16<INV>(v);
+    }
 }
 
-template <int M, typename InT, typename OutT>
-__global__ void __launch_bounds__(256, 3) filter_rf_kernel(const InT* __restrict__ raw, OutT* __restrict__ out,
-                                                           FilterArgs a, const float2* __restrict__ tw,
-                                                           const float* __restrict__ K) {
-    using C = RF<M>;
-    constexpr int L = C::L, L2 = C::L2, Q = C::Q;
-    extern __shared__ float2 smem[];
-    const int g = threadIdx.x / L, lt = threadIdx.x % L;
-    float2* sa = smem + g * C::SG;
-    const int W = a.W, H = a.H;
-    const int pairs = (H + 1) >> 1;
-    const long long q = (long long)blockIdx.x * C::G + g;
-    const bool active = q < a.n_views * pairs;
-    const long long view = active ? q / pairs : 0;
-    const int r0 = active ? int(q - view * pairs) * 2 : 0;
-    const bool has1 = active && r0 + 1 < H;
-    const InT* src = raw + (size_t)view * H * W + (size_t)r0 * W;
-    const float* wrow = a.wt + (size_t)r0 * W;
+__device__ __forceinline__ float4 as4(const C2& a) { return make_float4(a.x.x, a.x.y, a.y.x, a.y.y); }
+__device__ __forceinline__ C2 as2(const float4& a) { return {make_float2(a.x, a.y), make_float2(a.z, a.w)}; }
 
-    float2 v[16];
-    if (has1 && W == M) {
-        // whole row pair inside the detector: no per-column tests; the weights
-        // of the second row are loaded after the first row is done
-        InT x0[16], x1[16];
-        float wv[16];
+// -ln of two positive normal numbers. With m in [sqrt(1/2), sqrt(2)) the number's
+// mantissa, e its exponent and n = 1 - m (exact): -ln m = n + n^2 Q(n), Q a degree-8
+// least-maximum-error fit of the relative error over the interval (4e-9), and e ln 2
+// is taken off in two parts, the first exact for every e. Within about one unit in
+// the last place, as logf; the FP32x2 form shares each step between two samples.
+__device__ __forceinline__ float2 neg_ln2(float2 s) {
+    const int ix = __float_as_int(s.x) - 0x3F3504F3, iy = __float_as_int(s.y) - 0x3F3504F3;   // bits of sqrt(1/2)
+    const int ex = ix & 0xff800000, ey = iy & 0xff800000;                                     // e << 23
+    const float2 n = sub2(dup(1.0f), make_float2(__int_as_float(__float_as_int(s.x) - ex),
+                                                 __int_as_float(__float_as_int(s.y) - ey)));
+    // e as a float: 1.5 * 2^23 + e less the former
+    const float2 e = add2(make_float2(__int_as_float(0x4B400000 + (ix >> 23)), __int_as_float(0x4B400000 + (iy >> 23))),
+                          dup(-12582912.0f));
+    float2 q = dup(7.622107e-2f);
+    q = __ffma2_rn(q, n, dup(1.2904692e-1f));
+    q = __ffma2_rn(q, n, dup(1.3242977e-1f));
+    q = __ffma2_rn(q, n, dup(1.4181779e-1f));
+    q = __ffma2_rn(q, n, dup(1.6609077e-1f));
+    q = __ffma2_rn(q, n, dup(2.0001977e-1f));
+    q = __ffma2_rn(q, n, dup(2.5001583e-1f));
+    q = __ffma2_rn(q, n, dup(3.3333326e-1f));
+    q = __ffma2_rn(q, n, dup(4.9999988e-1f));
+    const float2 t = __ffma2_rn(__fmul2_rn(n, n), q, __fmul2_rn(e, dup(-1.4286068e-6f)));
+    return __ffma2_rn(e, dup(-0.693145752f), add2(n, t));   // 0.693145752 = 0xB1720 / 2^20
+}
+
+template <int M, bool HALF, typename InT, typename OutT>
+__global__ void __launch_bounds__(RF<M>::T, 512 / RF<M>::T)
+    filter_rf_kernel(const InT* __restrict__ raw, OutT* __restrict__ out, FilterArgs a, const float2* __restrict__ tw,
+                     const float* __restrict__ K, int plain_log) {
+    using C = RF<M>;
+    constexpr int L = C::L, L2 = C::L2, Q = C::Q, NR = HALF ? 8 : 16;
+    const float2* const tw1 = tw + M + threadIdx.x % L;              // pass 1: [s L]
+    const float2* const tw2 = tw + 2 * M + threadIdx.x % L % L2;     // pass 2: [s2 L2]
+    extern __shared__ float4 smem4[];
+    const int g = threadIdx.x / L, lt = threadIdx.x % L;
+    float4* sa = smem4 + g * C::SG;
+    const int W = a.W, H = a.H;
+    const int quads = (H + 3) >> 2;
+    const long long q = (long long)blockIdx.x * C::G + g;
+    const bool active = q < a.n_views * quads;
+    const long long view = active ? q / quads : 0;
+    const int r0 = active ? int(q - view * quads) * 4 : 0;
+    const int rows = active ? min(4, H - r0) : 0;
+    const InT* src = raw + ((size_t)view * H + r0) * W + lt;
+    const float* wrow = a.wt + (size_t)r0 * W + lt;
+
+    C2 v[16];
+    // rows ra and ra + 2 at once (the same component of the two signals)
+    auto load_rows = [&](auto rac, auto put) {
+        constexpr int ra = decltype(rac)::value;
+        InT x0[NR], x1[NR];
+        float w0[NR], w1[NR];
+        const bool has0 = ra < rows, has1 = ra + 2 < rows;
 #pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            x0[r] = src[lt + L * r];
-            x1[r] = src[W + lt + L * r];
-            wv[r] = __ldg(wrow + lt + L * r);
+        for (int r = 0; r < NR; ++r) {
+            const bool in = !HALF || lt + L * r < W;
+            x0[r] = in && has0 ? src[ra * W + L * r] : InT(1);
+            x1[r] = in && has1 ? src[(ra + 2) * W + L * r] : InT(1);
+            w0[r] = in && has0 ? __ldg(wrow + ra * W + L * r) : 0.0f;
+            w1[r] = in && has1 ? __ldg(wrow + (ra + 2) * W + L * r) : 0.0f;
         }
+        float2 p[NR];
 #pragma unroll
-        for (int r = 0; r < 16; ++r) v[r].x = __fmul_rn(log_part(raw_value(&x0[r], a), a), wv[r]);
+        for (int r = 0; r < NR; ++r)
+            p[r] = make_float2(__fmul_rn(raw_value(&x0[r], a), a.log_scale),
+                               __fmul_rn(raw_value(&x1[r], a), a.log_scale));
+        // whole-number samples of a positive base intensity are normal and positive; any
+        // other argument (zero, negative, tiny, infinite, NaN) goes to logf
+        bool odd = plain_log;
+        if constexpr (std::is_same<InT, float>::value) {
 #pragma unroll
-        for (int r = 0; r < 16; ++r) wv[r] = __ldg(wrow + W + lt + L * r);
-#pragma unroll
-        for (int r = 0; r < 16; ++r) v[r].y = __fmul_rn(log_part(raw_value(&x1[r], a), a), wv[r]);
-    } else {
-        // all 64 loads of the thread (16 columns x 2 rows, samples and weights)
-        // are issued before any arithmetic
-        InT x0[16], x1[16];
-        float w0[16], w1[16];
-#pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            const int c = lt + L * r;
-            const bool in = active && c < W;
-            x0[r] = in ? src[c] : InT(0);
-            x1[r] = in && has1 ? src[W + c] : InT(0);
-            w0[r] = in ? __ldg(wrow + c) : 0.0f;
-            w1[r] = in && has1 ? __ldg(wrow + W + c) : 0.0f;
+            for (int r = 0; r < NR; ++r)
+                odd |= unsigned(__float_as_int(p[r].x) - 0x00800000) >= 0x7f000000u ||
+                       unsigned(__float_as_int(p[r].y) - 0x00800000) >= 0x7f000000u;
         }
+        if (__builtin_expect(odd, 0)) {
 #pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            const int c = lt + L * r;
-            float2 z = make_float2(0.f, 0.f);
-            if (active && c < W) {
-                z.x = __fmul_rn(log_part(raw_value(&x0[r], a), a), w0[r]);
-                if (has1) z.y = __fmul_rn(log_part(raw_value(&x1[r], a), a), w1[r]);
+            for (int r = 0; r < NR; ++r) {
+                const float2 c = p[r];
+                p[r] = neg_ln2(c);
+                if (unsigned(__float_as_int(c.x) - 0x00800000) >= 0x7f000000u) p[r].x = -logf(c.x);
+                if (unsigned(__float_as_int(c.y) - 0x00800000) >= 0x7f000000u) p[r].y = -logf(c.y);
             }
-            v[r] = z;
+        } else {
+#pragma unroll
+            for (int r = 0; r < NR; ++r) p[r] = neg_ln2(p[r]);
         }
-    }
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            p[r] = __fmul2_rn(p[r], make_float2(w0[r], w1[r]));
+            if (!has0 || (HALF && lt + L * r >= W)) p[r].x = 0.0f;
+            if (!has1 || (HALF && lt + L * r >= W)) p[r].y = 0.0f;
+            put(r, p[r]);
+        }
+    };
+    load_rows(std::integral_constant<int, 0>{}, [&](int r, float2 p) { v[r].x = p; });
+    load_rows(std::integral_constant<int, 1>{}, [&](int r, float2 p) { v[r].y = p; });
+
     // pass 1
-    dft16<false>(v);
+    dft16<false, HALF>(v);
 #pragma unroll
-    for (int s = 1; s < 16; ++s) v[s] = cmul(v[s], __ldg(&tw[lt * s]));
+    for (int s = 1; s < 16; ++s) v[s] = mul2<false>(v[s], __ldg(tw1 + s * L));
 #pragma unroll
-    for (int s = 0; s < 16; ++s) sa[s * (L + L2) + lt] = v[s];
+    for (int s = 0; s < 16; ++s) sa[s * (L + L2) + lt] = as4(v[s]);
     __syncthreads();
     // pass 2
     const int ps = lt / L2, t2 = lt % L2;
-    float2* bs = sa + (C::ALIAS ? 0 : C::SA) + ps * C::SB;
+    float4* bs = sa + ps * C::SB;
 #pragma unroll
-    for (int r = 0; r < 16; ++r) v[r] = sa[ps * (L + L2) + t2 + L2 * r];
+    for (int r = 0; r < 16; ++r) v[r] = as2(sa[ps * (L + L2) + t2 + L2 * r]);
     dft16<false>(v);
+    if constexpr (L2 == 1) {
+        // X[s + 16 s2] is here
 #pragma unroll
-    for (int s2 = 1; s2 < 16; ++s2) v[s2] = cmul(v[s2], __ldg(&tw[16 * t2 * s2]));
-    if (C::ALIAS) __syncthreads();  // the second transpose overwrites the first
-#pragma unroll
-    for (int s2 = 0; s2 < 16; ++s2) bs[s2 * (L2 + 1) + t2] = v[s2];
-    __syncwarp();
-    // pass 3, the kernel spectrum, inverse pass 3
-    {
-        float2 u[Q][L2];
-#pragma unroll
-        for (int qq = 0; qq < Q; ++qq)
-#pragma unroll
-            for (int k = 0; k < L2; ++k) u[qq][k] = bs[(t2 + L2 * qq) * (L2 + 1) + k];
-#pragma unroll
-        for (int qq = 0; qq < Q; ++qq) {
-            dft_n<L2, false>(u[qq]);
-#pragma unroll
-            for (int k3 = 0; k3 < L2; ++k3) {
-                const float kf = __ldg(&K[ps + 16 * (t2 + L2 * qq) + 256 * k3]);
-                u[qq][k3] = make_float2(u[qq][k3].x * kf, u[qq][k3].y * kf);
-            }
-            dft_n<L2, true>(u[qq]);
+        for (int s2 = 0; s2 < 16; ++s2) {
+            const float2 k = dup(__ldg(&K[ps + 16 * s2]));
+            v[s2] = {__fmul2_rn(v[s2].x, k), __fmul2_rn(v[s2].y, k)};
         }
-        __syncwarp();
+    } else {
 #pragma unroll
-        for (int qq = 0; qq < Q; ++qq)
+        for (int s2 = 1; s2 < 16; ++s2) v[s2] = mul2<false>(v[s2], __ldg(tw2 + s2 * L2));
+        __syncthreads();  // the second transpose overwrites the first
 #pragma unroll
-            for (int k = 0; k < L2; ++k) bs[(t2 + L2 * qq) * (L2 + 1) + k] = u[qq][k];
+        for (int s2 = 0; s2 < 16; ++s2) bs[s2 * (L2 + 1) + t2] = as4(v[s2]);
         __syncwarp();
+        // pass 3, the kernel spectrum, inverse pass 3
+        {
+            C2 u[Q][L2];
+#pragma unroll
+            for (int qq = 0; qq < Q; ++qq)
+#pragma unroll
+                for (int k = 0; k < L2; ++k) u[qq][k] = as2(bs[(t2 + L2 * qq) * (L2 + 1) + k]);
+#pragma unroll
+            for (int qq = 0; qq < Q; ++qq) {
+                dft_n<L2, false>(u[qq]);
+#pragma unroll
+                for (int k3 = 0; k3 < L2; ++k3) {
+                    const float2 kf = dup(__ldg(&K[ps + 16 * (t2 + L2 * qq) + 256 * k3]));
+                    u[qq][k3] = {__fmul2_rn(u[qq][k3].x, kf), __fmul2_rn(u[qq][k3].y, kf)};
+                }
+                dft_n<L2, true>(u[qq]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int qq = 0; qq < Q; ++qq)
+#pragma unroll
+                for (int k = 0; k < L2; ++k) bs[(t2 + L2 * qq) * (L2 + 1) + k] = as4(u[qq][k]);
+            __syncwarp();
+        }
+        // inverse pass 2
+#pragma unroll
+        for (int s2 = 0; s2 < 16; ++s2) v[s2] = as2(bs[s2 * (L2 + 1) + t2]);
+#pragma unroll
+        for (int s2 = 1; s2 < 16; ++s2) v[s2] = mul2<true>(v[s2], __ldg(tw2 + s2 * L2));
     }
-    // inverse pass 2
-#pragma unroll
-    for (int s2 = 0; s2 < 16; ++s2) v[s2] = bs[s2 * (L2 + 1) + t2];
-#pragma unroll
-    for (int s2 = 1; s2 < 16; ++s2) v[s2] = cmul_conj(v[s2], __ldg(&tw[16 * t2 * s2]));
     dft16<true>(v);
-    __syncthreads();  // every warp has read its pass-2 values from sa
+    __syncthreads();  // every warp has read its values of the transpose before
 #pragma unroll
-    for (int r = 0; r < 16; ++r) sa[ps * (L + L2) + t2 + L2 * r] = v[r];
+    for (int r = 0; r < 16; ++r) sa[ps * (L + L2) + t2 + L2 * r] = as4(v[r]);
     __syncthreads();
     // inverse pass 1 and the filtered rows
 #pragma unroll
-    for (int s = 0; s < 16; ++s) v[s] = sa[s * (L + L2) + lt];
+    for (int s = 0; s < 16; ++s) v[s] = as2(sa[s * (L + L2) + lt]);
 #pragma unroll
-    for (int s = 1; s < 16; ++s) v[s] = cmul_conj(v[s], __ldg(&tw[lt * s]));
-    dft16<true>(v);
-    const size_t obase = (size_t)view * H * a.out_pitch + (size_t)r0 * a.out_pitch;
+    for (int s = 1; s < 16; ++s) v[s] = mul2<true>(v[s], __ldg(tw1 + s * L));
+    dft16<true, false, HALF>(v);
+    OutT* const dst = out + ((size_t)view * H + r0) * a.out_pitch + lt;
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
-        const int c = lt + L * r;
-        if (active && c < W) {
-            out[obase + c] = to_store<OutT>(v[r].x * a.store_scale);
-            if (has1) out[obase + a.out_pitch + c] = to_store<OutT>(v[r].y * a.store_scale);
-        }
+    for (int r = 0; r < NR; ++r) {
+        if (HALF && lt + L * r >= W) continue;
+        const float e[4] = {v[r].x.x, v[r].y.x, v[r].x.y, v[r].y.y};   // rows r0 .. r0 + 3
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (k < rows) dst[(size_t)k * a.out_pitch + L * r] = to_store<OutT>(e[k] * a.store_scale);
     }
 }
 
-template <int M, typename InT, typename OutT>
+template <int M, bool HALF, typename InT, typename OutT>
 int launch_rf(const InT* raw, OutT* out, const FilterArgs& a, const float2* tw, const float* K, cudaStream_t s) {
     using C = RF<M>;
-    const long long pairs = a.n_views * ((a.H + 1) / 2);
-    const long long blocks = (pairs + C::G - 1) / C::G;
+    const long long quads = a.n_views * ((a.H + 3) / 4);
+    const long long blocks = (quads + C::G - 1) / C::G;
     if (blocks <= 0) return CTB_OK;
     if (blocks > 0x7fffffffLL) {
         set_global_error("filter: too many rows for one launch");
         return CTB_ERR_UNSUPPORTED;
     }
-    const size_t smem = size_t(C::G) * C::SG * sizeof(float2);
-    auto kern = filter_rf_kernel<M, InT, OutT>;
+    const size_t smem = size_t(C::G) * C::SG * sizeof(float4);
+    auto kern = filter_rf_kernel<M, HALF, InT, OutT>;
     if (const int st = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) return st;
-    kern<<<unsigned(blocks), 256, smem, s>>>(raw, out, a, tw, K);
+    // samples of 8 and 16 bits give arguments from beta to (1 + beta) times the scale
+    const bool normal = a.beta > 0.0f && a.log_scale > 0.0f && a.beta * a.log_scale > 1e-30f && a.log_scale < 1e30f;
+    kern<<<unsigned(blocks), C::T, smem, s>>>(raw, out, a, tw, K, !std::is_same<InT, float>::value && !normal);
     return cuda_status(cudaGetLastError(), "filter_rf_kernel launch");
+}
+
+// whole rows of a power-of-two width, or rows embedded in a transform at least twice as long
+template <int M, typename InT, typename OutT>
+int launch_rf_any(const InT* raw, OutT* out, const FilterArgs& a, const float2* tw, const float* K, cudaStream_t s) {
+    return a.W == M ? launch_rf<M, false>(raw, out, a, tw, K, s) : launch_rf<M, true>(raw, out, a, tw, K, s);
 }
 
 template <typename InT, typename OutT>
@@ -616,12 +757,13 @@ int launch_typed(const InT* raw, OutT* out, const FilterArgs& a, const float2* t
         return CTB_ERR_UNSUPPORTED;
     }
     const bool tab = a.wt != nullptr;
-    if (tab) {
+    if (tab && (a.W == a.M || 2 * a.W <= a.M)) {
         switch (a.M) {
-            case 512: return launch_rf<512>(raw, out, a, tw, K, s);
-            case 1024: return launch_rf<1024>(raw, out, a, tw, K, s);
-            case 2048: return launch_rf<2048>(raw, out, a, tw, K, s);
-            case 4096: return launch_rf<4096>(raw, out, a, tw, K, s);
+            case 256: return launch_rf_any<256>(raw, out, a, tw, K, s);
+            case 512: return launch_rf_any<512>(raw, out, a, tw, K, s);
+            case 1024: return launch_rf_any<1024>(raw, out, a, tw, K, s);
+            case 2048: return launch_rf_any<2048>(raw, out, a, tw, K, s);
+            case 4096: return launch_rf_any<4096>(raw, out, a, tw, K, s);
         }
     }
     auto kern = tab ? filter_kernel<InT, OutT, true> : filter_kernel<InT, OutT, false>;
@@ -655,10 +797,16 @@ int filter_transform_length(int W, int pad) {
     return M > kMaxFftLen ? 0 : int(M);
 }
 
+int filter_twiddle_count(int M) { return M >= 256 && M <= 4096 ? 2 * M + M / 16 : M; }
+
 int filter_build_tables(int W, int pad, int filter, int M, float2* tw, float* K, cudaStream_t s) {
     const int T = 256;
     twiddle_kernel<<<(M + T - 1) / T, T, 0, s>>>(tw, M);
     CTB_CUDA_TRY(cudaGetLastError());
+    if (filter_twiddle_count(M) > M) {
+        twiddle_order_kernel<<<(M + M / 16 + T - 1) / T, T, 0, s>>>(tw, M);
+        CTB_CUDA_TRY(cudaGetLastError());
+    }
     if (pad >= 2) {
         kernel_padded<<<(M + T - 1) / T, T, 0, s>>>(K, M, W, filter);
     } else if (M == W) {
