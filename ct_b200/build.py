@@ -37,6 +37,7 @@ SOURCES = [
     "kernels/layout.cu",
     "kernels/phantom.cu",
     "host/errors.cpp",
+    "host/scratch.cpp",
     "host/image_io.cpp",
     "host/reconstructor.cpp",
     "host/volume_io.cpp",

@@ -29,18 +29,8 @@ int arg_error(const char* msg) {
 
 // Device view table {sin, cos, h} from host angle / height arrays.
 int upload_views(const double* ang, const double* h, int n, cudaStream_t s, float4** views) {
-    double* d = nullptr;
-    CTB_CUDA_TRY(cudaMallocAsync((void**)&d, sizeof(double) * 2 * n, s));
-    CTB_CUDA_TRY(cudaMallocAsync((void**)views, sizeof(float4) * n, s));
-    CTB_CUDA_TRY(cudaMemcpyAsync(d, ang, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    if (h) {
-        CTB_CUDA_TRY(cudaMemcpyAsync(d + n, h, sizeof(double) * n, cudaMemcpyHostToDevice, s));
-    } else {
-        CTB_CUDA_TRY(cudaMemsetAsync(d + n, 0, sizeof(double) * n, s));
-    }
-    int st = ctb::view_table_build(d, d + n, n, *views, s);
-    CTB_CUDA_TRY(cudaFreeAsync(d, s));
-    return st;
+    CTB_CUDA_TRY(ctb::scratch_alloc((void**)views, sizeof(float4) * n, s));
+    return ctb::view_table_from_host(ang, h, n, *views, s);
 }
 
 }  // namespace

@@ -31,6 +31,18 @@ int cuda_status(cudaError_t e, const char* what);
 // invalidated by another thread lowering it.
 int ensure_dynamic_smem(const void* kernel, size_t bytes);
 
+// Device memory of one operator call, given back with cudaFreeAsync on the same
+// stream: from the library's pool of the current device (host/scratch.cpp), from
+// the stream's graph while it is captured.
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s);
+// Give the pool's unused memory of the current device back to the driver.
+void scratch_trim();
+// cudaMalloc, tried again after scratch_trim when memory is short.
+cudaError_t device_alloc(void** p, size_t bytes);
+// Unique ID of the current context (0 when it cannot be told: no context
+// current yet, or a driver without cuCtxGetId).
+unsigned long long current_context_id();
+
 // Argument checks shared by the operator entry points.
 inline bool valid_detector(const ctb_detector* d) {
     return d && d->width > 1 && d->height > 1 && d->fcd > float(d->width) && d->base_intensity != 0.0f;
@@ -107,6 +119,8 @@ FilterArgs filter_args(const ctb_detector& det, int raw_type, int M, int logM, l
 // of that float in double precision, rounded to float (Ct/CtVolume.cpp:953-955).
 int view_table_build(const double* angles_deg_dev, const double* heights_dev, int n, float4* out,
                      cudaStream_t s);
+// The same from host arrays (heights may be null: zeros), read before it returns.
+int view_table_from_host(const double* angles_deg, const double* heights, int n, float4* out, cudaStream_t s);
 
 // Constants of one backprojection / forward projection launch (slab-local).
 struct ProjGeom {

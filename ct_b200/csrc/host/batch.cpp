@@ -149,7 +149,7 @@ int ctb_batch_create(ctb_batch** out, int n, const ctb_scan* scans, int store_ty
         const int pitch = (sc.det.width + 7) / 8 * 8;
         b->pitch.push_back(pitch);
         void* f = nullptr;
-        if (cudaMalloc(&f, es * size_t(sc.n_views) * sc.det.height * pitch) != cudaSuccess) {
+        if (device_alloc(&f, es * size_t(sc.n_views) * sc.det.height * pitch) != cudaSuccess) {
             cudaGetLastError();
             return bail(fail("ctb_batch_create: out of device memory for filtered projections", CTB_ERR_ALLOC));
         }

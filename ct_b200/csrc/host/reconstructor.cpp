@@ -55,7 +55,7 @@ int DevBuf::ensure(size_t n, const char* what) {
                          " failed (injected)");
         return CTB_ERR_ALLOC;
     }
-    cudaError_t e = cudaMalloc(&p, n);
+    cudaError_t e = device_alloc(&p, n);
     if (e != cudaSuccess) {
         p = nullptr;
         cudaGetLastError();
@@ -815,7 +815,8 @@ int Reconstructor::run_pipeline(DeviceWork& w, float* out, int order, int z_lo, 
     const size_t view_filt = size_t(pitch) * Hb * store_bytes(store_);
     const int chunk = int(std::max<size_t>(1, std::min<size_t>(size_t(V), (size_t(256) << 20) / view_raw)));
     const size_t plane = size_t(X) * Y;
-    // default: about a quarter of the slices per slab, a multiple of 16 (1440
+    // default: about a quarter of the slices per slab, a multiple of 32 (whole
+    // tiles; 192 slices of the 360-view 256 x 192 scan in slabs of 64, not 48; 1440
     // views of 2048^2 into 1024^3, end to end: 256 slices 0.6 % faster than
     // 128, fewer launch tails, while two slabs still cover the upload and the
     // cut last slab keeps the final download short)
@@ -823,10 +824,11 @@ int Reconstructor::run_pipeline(DeviceWork& w, float* out, int order, int z_lo, 
     BpConfig bpc;
     int tuned_slab = 0;
     const bool tuned = tuned_for(z_lo, z_hi, &bpc, &tuned_slab);
-    int slab = slab_req_ > 0 ? slab_req_ : tuned ? tuned_slab : std::max(16, ((Zw + 3) / 4 + 15) / 16 * 16);
+    int slab = slab_req_ > 0 ? slab_req_ : tuned ? tuned_slab : std::max(32, ((Zw + 3) / 4 + 31) / 32 * 32);
     slab = std::min(slab, Zw);
     const bool convert = order == CTB_Z_FASTEST;
     {
+        scratch_trim();   // (what the operators' pool holds counts as free)
         size_t freeb = 0, total = 0;
         cudaMemGetInfo(&freeb, &total);
         const size_t spare = spare_mb_ << 20;

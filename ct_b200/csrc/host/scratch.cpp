@@ -1,0 +1,131 @@
+// Device memory that one operator call takes and gives back on its stream (view
+// tables, the projector's volume copy, repacked rows): a stream-ordered pool per
+// device that keeps up to kKeep bytes between calls. The device's default pool
+// returns everything at each synchronisation, so that a program that waits for
+// every call paid for mapping memory again each time (120 views of 200 x 150 into
+// 96^3, filter and backprojection, each call waited for: 4.8 ms, with this pool 0.18
+// ms; the smallest scan, 24 views of 32 x 20, 0.51 and 0.058 ms). The pool is the
+// library's own: no setting of the default pool changes for the rest of the
+// process. It is emptied when an allocation of the library fails, before that is
+// tried again.
+
+#include <cuda.h>
+#include <cuda_runtime.h>
+
+#include <cstdint>
+#include <map>
+#include <mutex>
+
+#include "../ctb_internal.h"
+
+namespace ctb {
+
+unsigned long long current_context_id() {
+    using GetCurrent = CUresult (*)(CUcontext*);
+    using GetId = CUresult (*)(CUcontext, unsigned long long*);
+    static GetCurrent get_current = nullptr;
+    static GetId get_id = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* a = nullptr;
+        void* b = nullptr;
+        cudaDriverEntryPointQueryResult qa, qb;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &a, cudaEnableDefault, &qa) == cudaSuccess &&
+            qa == cudaDriverEntryPointSuccess &&
+            cudaGetDriverEntryPoint("cuCtxGetId", &b, cudaEnableDefault, &qb) == cudaSuccess &&
+            qb == cudaDriverEntryPointSuccess) {
+            get_current = reinterpret_cast<GetCurrent>(a);
+            get_id = reinterpret_cast<GetId>(b);
+        } else {
+            cudaGetLastError();
+        }
+    });
+    CUcontext c = nullptr;
+    unsigned long long id = 0;
+    if (!get_current || get_current(&c) != CUDA_SUCCESS || !c || get_id(c, &id) != CUDA_SUCCESS) return 0;
+    return id;
+}
+
+namespace {
+
+constexpr uint64_t kKeep = uint64_t(256) << 20;
+
+struct Pool {
+    cudaMemPool_t pool = nullptr;
+    unsigned long long ctx = 0;   // the context the pool belongs to
+};
+std::mutex g_pool_mtx;
+std::map<int, Pool> g_pools;
+
+// The current device's pool (null: none to be had, or a capturing stream, whose
+// allocations belong to its graph).
+cudaMemPool_t scratch_pool(cudaStream_t s) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    const unsigned long long ctx = current_context_id();
+    if (ctx == 0) return nullptr;
+    std::lock_guard<std::mutex> lk(g_pool_mtx);
+    Pool& p = g_pools[dev];
+    if (p.pool && p.ctx == ctx) return p.pool;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    uint64_t keep = kKeep;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
+    p.pool = pool;   // (a pool of a context that is gone went with it)
+    p.ctx = ctx;
+    return pool;
+}
+
+}  // namespace
+
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t s) {
+    cudaMemPool_t pool = scratch_pool(s);
+    if (!pool) return cudaMallocAsync(p, bytes, s);
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        scratch_trim();
+        e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+    }
+    return e;
+}
+
+void scratch_trim() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    const unsigned long long ctx = current_context_id();
+    std::lock_guard<std::mutex> lk(g_pool_mtx);
+    auto it = g_pools.find(dev);
+    if (it == g_pools.end() || !it->second.pool || it->second.ctx != ctx) return;
+    if (cudaMemPoolTrimTo(it->second.pool, 0) != cudaSuccess) cudaGetLastError();
+}
+
+cudaError_t device_alloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        scratch_trim();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
+}  // namespace ctb

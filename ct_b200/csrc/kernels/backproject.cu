@@ -33,15 +33,39 @@ namespace ctb {
 
 namespace {
 
+__device__ __forceinline__ float4 view_record(double ang, double h) {
+    // float angle_rad = (angle / 180.0) * M_PI; sine = sin(angle_rad) (:953-955)
+    const float angle_rad = float((ang / 180.0) * 3.14159265358979323846);
+    double s, c;
+    sincos(double(angle_rad), &s, &c);
+    return make_float4(float(s), float(c), float(h), 0.0f);
+}
+
 __global__ void view_table_kernel(const double* __restrict__ ang, const double* __restrict__ h, int n,
                                   float4* __restrict__ out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    // float angle_rad = (angle / 180.0) * M_PI; sine = sin(angle_rad) (:953-955)
-    const float angle_rad = float((ang[i] / 180.0) * 3.14159265358979323846);
-    double s, c;
-    sincos(double(angle_rad), &s, &c);
-    out[i] = make_float4(float(s), float(c), float(h[i]), 0.0f);
+    if (i < n) out[i] = view_record(ang[i], h[i]);
+}
+
+// N views' angles and heights as kernel arguments: no device copy of the host
+// arrays to allocate, fill and give back (a call of the smallest scans spent more
+// host time on those than on its launches).
+template <int N> struct HostViews {
+    double ang[N], h[N];
+};
+template <int N>
+__global__ void view_table_args_kernel(const __grid_constant__ HostViews<N> v, int n, float4* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = view_record(v.ang[i], v.h[i]);
+}
+
+template <int N>
+void view_table_args(const double* ang, const double* h, int n, float4* out, cudaStream_t s) {
+    HostViews<N> v;
+    std::memcpy(v.ang, ang, sizeof(double) * n);
+    if (h) std::memcpy(v.h, h, sizeof(double) * n);
+    else std::memset(v.h, 0, sizeof(double) * n);
+    view_table_args_kernel<N><<<(n + 127) / 128, 128, 0, s>>>(v, n, out);
 }
 
 template <typename T> __device__ __forceinline__ float ld(const T* p);
@@ -166,6 +190,17 @@ int view_table_build(const double* angles_deg_dev, const double* heights_dev, in
     return cuda_status(cudaGetLastError(), "view_table_kernel launch");
 }
 
+int view_table_from_host(const double* angles_deg, const double* heights, int n, float4* out, cudaStream_t s) {
+    constexpr int kMost = 1024;   // 16 KB of arguments a launch
+    for (int i = 0; i < n; i += kMost) {
+        const int k = std::min(kMost, n - i);
+        const double* h = heights ? heights + i : nullptr;
+        if (k <= 128) view_table_args<128>(angles_deg + i, h, k, out + i, s);
+        else view_table_args<kMost>(angles_deg + i, h, k, out + i, s);
+    }
+    return cuda_status(cudaGetLastError(), "view_table_args_kernel launch");
+}
+
 static inline float __fmul_rn_host(float a, float b) { return a * b; }
 
 ProjGeom proj_geom(const ctb_detector& det, const ctb_grid& grid, int z_begin, int z_end, float load_scale) {
@@ -278,7 +313,7 @@ int backproject_repacked(const void* proj, int store_type, const float4* views, 
     const size_t cap = std::max(size_t(256) << 20, sizeof(float) * size_t(g.X) * g.Y * g.Zs);
     const int run = int(std::max<size_t>(1, std::min<size_t>(size_t(n_views), cap / view_bytes)));
     void* rows = nullptr;
-    if (cudaMallocAsync(&rows, view_bytes * run, s) != cudaSuccess) {
+    if (scratch_alloc(&rows, view_bytes * run, s) != cudaSuccess) {
         cudaGetLastError();
         return CTB_ERR_UNSUPPORTED;
     }

@@ -760,17 +760,30 @@ bool box_dims(const ProjGeom& g, int ZC, double hmax, int esize, Box* b) {
     // T U sqrt(1 + (t U / D)^2) to first order; the second-order terms
     // (|u_ss| = 2 |t| U^3 / D^2, |u_st| = U^2 / D) add at most
     // (T/2)^2 (|u_ss| + 2 |u_st|) / 2. For each s the largest |t| within R
-    // of the axis is the worst; s is scanned finely (the extent changes by
-    // far less than 0.05 pixel between samples). Views whose footprint still
+    // of the axis is the worst; s is scanned (the extent changes by far less
+    // than 0.05 pixel between the finest samples). Views whose footprint still
     // does not fit are read through global memory by the kernel.
-    double uext = 0.0;
-    for (int i = 0; i <= 4096; ++i) {
-        const double s = R * (2.0 * i / 4096 - 1.0);
+    auto extent = [&](double s) {
         const double t = std::sqrt(std::max(0.0, R * R - s * s)) + std::fabs(g.uOff);
         const double U = D / (D - s);
         const double first = T * U * std::sqrt(1.0 + (t * U / D) * (t * U / D));
         const double second = 0.125 * T * T * (2.0 * t * U * U * U / (D * D) + 2.0 * U * U / D);
-        uext = std::max(uext, first + second);
+        return first + second;
+    };
+    // (coarse, then finely around the largest: the extent is smooth in s but for its
+    // root at the ends, which the fine steps resolve)
+    double uext = 0.0;
+    int at = 0;
+    for (int i = 0; i <= 128; ++i) {
+        const double e = extent(R * (2.0 * i / 128 - 1.0));
+        if (e > uext) {
+            uext = e;
+            at = i;
+        }
+    }
+    for (int k = -32; k <= 32; ++k) {
+        const double s = R * (2.0 * (at + k / 32.0) / 128 - 1.0);
+        if (std::fabs(s) <= R) uext = std::max(uext, extent(s));
     }
     uext += 0.05;
     const double zabs =

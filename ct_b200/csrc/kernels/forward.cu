@@ -404,7 +404,7 @@ int forward_launch(const float* vol, const float4* views, int n_views, const Pro
     // z-fastest scratch copy of the slab, the flag before it
     const size_t n = size_t(g.X) * g.Y * g.Zs;
     char* scratch = nullptr;
-    CTB_CUDA_TRY(cudaMallocAsync((void**)&scratch, 256 + sizeof(float) * n, s));
+    CTB_CUDA_TRY(scratch_alloc((void**)&scratch, 256 + sizeof(float) * n, s));
     int* nonfinite = reinterpret_cast<int*>(scratch);
     float* volz = reinterpret_cast<float*>(scratch + 256);
     int st = cuda_status(cudaMemsetAsync(nonfinite, 0, sizeof(int), s), "forward projector flag");

@@ -33,7 +33,6 @@
 //    (different streams, or concurrent host threads on the same device) race
 //    on it: serialise them.
 
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -55,34 +54,6 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 std::mutex g_addr_mtx;
 void* g_addr[kMaxDevices] = {};
 unsigned long long g_ctx_id[kMaxDevices] = {};
-
-// Unique ID of the current context (0 when it cannot be told: no context
-// current yet, or a driver without cuCtxGetId).
-unsigned long long current_context_id() {
-    using GetCurrent = CUresult (*)(CUcontext*);
-    using GetId = CUresult (*)(CUcontext, unsigned long long*);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* a = nullptr;
-        void* b = nullptr;
-        cudaDriverEntryPointQueryResult qa, qb;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &a, cudaEnableDefault, &qa) == cudaSuccess &&
-            qa == cudaDriverEntryPointSuccess &&
-            cudaGetDriverEntryPoint("cuCtxGetId", &b, cudaEnableDefault, &qb) == cudaSuccess &&
-            qb == cudaDriverEntryPointSuccess) {
-            get_current = reinterpret_cast<GetCurrent>(a);
-            get_id = reinterpret_cast<GetId>(b);
-        } else {
-            cudaGetLastError();
-        }
-    });
-    CUcontext c = nullptr;
-    unsigned long long id = 0;
-    if (!get_current || get_current(&c) != CUDA_SUCCESS || !c || get_id(c, &id) != CUDA_SUCCESS) return 0;
-    return id;
-}
 
 // Device address of the scratch array on the current device: looked up once
 // per device (and again if the device's context was replaced).
