@@ -96,17 +96,22 @@ template <> __device__ __forceinline__ float sval<__nv_bfloat16>(__nv_bfloat16 v
 
 // The fast column loop on pairs of voxels (j, j + 1) with the FP32x2
 // instructions of sm_100 (one issue slot for two lanes' worth of FFMA/FADD).
-// Same operations and roundings as the scalar loop, so the sums are
+// Same operations and roundings as the other loops (masked, global memory), so the sums are
 // bit-identical: the row floor is taken by adding 1.5 * 2^23 rounded toward
 // zero (exact for 0 <= vi < 2^22; the caller guarantees vi >= 0.5), whose low
 // bits are the row index and whose difference from the magic is float(v0);
-// subtractions are FMAs with a -1 factor (one rounding, as a subtraction).
+// subtractions are FMAs with a -1 factor (one rounding, as a subtraction). The
+// interpolation runs along the rows first, then the two columns are summed with
+// their weights w (1-fu) and w fu, which a column has once per view: one FP32x2
+// operation per pair less than interpolating along u and weighting the result (720
+// views of 1024^2 into 512^3: FP32 56.0 -> 54.7 ms, FP16 56.2 -> 54.1, BF16 54.2 -> 52.5;
+// 360 of 256 x 192 into 256^3 FP32 3.26 -> 3.14).
 // Rows of the box relative to its origin row, for the bounds-checked build.
 struct BoxRows {
     int oy, BV;
 };
 
-// float(b) - a for a stored texel b and an FP32 a. For the 16-bit types one
+// float(b) - a for a stored texel b (of row v0 + 1) and an FP32 a. For the 16-bit types one
 // mixed-precision instruction of sm_100 (sub.rn.f32.f16 / .bf16) converts b
 // and subtracts: the same value as the conversion followed by the subtraction
 // (the conversion is exact, one rounding), one instruction instead of a
@@ -141,7 +146,8 @@ __device__ __forceinline__ void column_pairs(const T* col, const int BU_run, con
     static_assert(OFF % ZC == 0 && OFF + ZC <= 32, "a tile lies inside one block of 32 slices");
     const int BU = KBU > 0 ? KBU : BU_run;
     constexpr float kMagic = 12582912.0f;   // 1.5 * 2^23
-    const float2 fu2 = make_float2(fu, fu), w2 = make_float2(w, w);
+    const float wa = w * (1.0f - fu), wb = w * fu;   // of columns u0, u0 + 1
+    const float2 wa2 = make_float2(wa, wa), wb2 = make_float2(wb, wb);
     const float2 m1 = make_float2(-1.0f, -1.0f), mg = make_float2(kMagic, kMagic);
     const float2 mdv2 = make_float2(mdv, mdv), c0b2 = make_float2(c0b, c0b);
 #pragma unroll
@@ -162,19 +168,18 @@ __device__ __forceinline__ void column_pairs(const T* col, const int BU_run, con
         const T* ra = col + rowa * BU;
         const T* rb = col + rowb * BU;
         const float2 p00 = make_float2(sval(ra[0]), sval(rb[0]));
-        const float2 p10 = make_float2(sval(ra[BU]), sval(rb[BU]));
-        float2 d0, d1;   // p01 - p00, p11 - p10
+        const float2 p01 = make_float2(sval(ra[1]), sval(rb[1]));
+        float2 d0, d1;   // p10 - p00, p11 - p01
         if constexpr (sizeof(T) == 4) {
-            d0 = __ffma2_rn(p00, m1, make_float2(sval(ra[1]), sval(rb[1])));
-            d1 = __ffma2_rn(p10, m1, make_float2(sval(ra[BU + 1]), sval(rb[BU + 1])));
+            d0 = __ffma2_rn(p00, m1, make_float2(sval(ra[BU]), sval(rb[BU])));
+            d1 = __ffma2_rn(p01, m1, make_float2(sval(ra[BU + 1]), sval(rb[BU + 1])));
         } else {
-            d0 = make_float2(sub_from(ra[1], p00.x), sub_from(rb[1], p00.y));
-            d1 = make_float2(sub_from(ra[BU + 1], p10.x), sub_from(rb[BU + 1], p10.y));
+            d0 = make_float2(sub_from(ra[BU], p00.x), sub_from(rb[BU], p00.y));
+            d1 = make_float2(sub_from(ra[BU + 1], p01.x), sub_from(rb[BU + 1], p01.y));
         }
-        const float2 a = __ffma2_rn(fu2, d0, p00);
-        const float2 c = __ffma2_rn(fu2, d1, p10);
-        const float2 r = __ffma2_rn(fv, __ffma2_rn(a, m1, c), a);
-        const float2 s = __ffma2_rn(w2, r, make_float2(acc[j], acc[j + 1]));
+        const float2 q0 = __ffma2_rn(fv, d0, p00);
+        const float2 q1 = __ffma2_rn(fv, d1, p01);
+        const float2 s = __ffma2_rn(wb2, q1, __ffma2_rn(wa2, q0, make_float2(acc[j], acc[j + 1])));
         acc[j] = s.x;
         acc[j + 1] = s.y;
     }
@@ -189,7 +194,8 @@ template <typename T, int N>
 __device__ __forceinline__ void column_pairs_masked(const T* col, const int BU, float fzo, float c0b, float mdv,
                                                     float fu, float w, unsigned in, float* acc, BoxRows br) {
     constexpr float kMagic = 12582912.0f;   // 1.5 * 2^23
-    const float2 fu2 = make_float2(fu, fu), w2 = make_float2(w, w);
+    const float wa = w * (1.0f - fu), wb = w * fu;
+    const float2 wa2 = make_float2(wa, wa), wb2 = make_float2(wb, wb);
     const float2 m1 = make_float2(-1.0f, -1.0f), mg = make_float2(kMagic, kMagic);
 #pragma unroll
     for (int j = 0; j < N; j += 2) {
@@ -208,13 +214,12 @@ __device__ __forceinline__ void column_pairs_masked(const T* col, const int BU, 
         const T* ra = col + rowa * BU;
         const T* rb = col + rowb * BU;
         const float2 p00 = make_float2(sval(ra[0]), sval(rb[0]));
-        const float2 p10 = make_float2(sval(ra[BU]), sval(rb[BU]));
-        const float2 d0 = make_float2(sub_from(ra[1], p00.x), sub_from(rb[1], p00.y));
-        const float2 d1 = make_float2(sub_from(ra[BU + 1], p10.x), sub_from(rb[BU + 1], p10.y));
-        const float2 a = __ffma2_rn(fu2, d0, p00);
-        const float2 c = __ffma2_rn(fu2, d1, p10);
-        const float2 r = __ffma2_rn(fv, __ffma2_rn(a, m1, c), a);
-        const float2 s = __ffma2_rn(w2, r, make_float2(acc[j], acc[j + 1]));
+        const float2 p01 = make_float2(sval(ra[1]), sval(rb[1]));
+        const float2 d0 = make_float2(sub_from(ra[BU], p00.x), sub_from(rb[BU], p00.y));
+        const float2 d1 = make_float2(sub_from(ra[BU + 1], p01.x), sub_from(rb[BU + 1], p01.y));
+        const float2 q0 = __ffma2_rn(fv, d0, p00);
+        const float2 q1 = __ffma2_rn(fv, d1, p01);
+        const float2 s = __ffma2_rn(wb2, q1, __ffma2_rn(wa2, q0, make_float2(acc[j], acc[j + 1])));
         if (ina) acc[j] = s.x;
         if (inb) acc[j + 1] = s.y;
     }
@@ -529,9 +534,10 @@ __device__ __forceinline__ bool tile_pass(const CUtensorMap* map, const T* __res
                             if (!CTB_FETCH_OK(v0, g.H - 1, 4)) v0 = 0;
 #endif
                             const T* r0 = col + (long long)v0 * g.pitch;
-                            const float a = fmaf(fu, gval(r0 + 1) - gval(r0), gval(r0));
-                            const float c = fmaf(fu, gval(r0 + g.pitch + 1) - gval(r0 + g.pitch), gval(r0 + g.pitch));
-                            acc[j] = fmaf(w, fmaf(fv, c - a, a), acc[j]);
+                            const float p00 = gval(r0), p01 = gval(r0 + 1);
+                            const float q0 = fmaf(fv, __fsub_rn(gval(r0 + g.pitch), p00), p00);
+                            const float q1 = fmaf(fv, __fsub_rn(gval(r0 + g.pitch + 1), p01), p01);
+                            acc[j] = fmaf(w * fu, q1, fmaf(w * (1.0f - fu), q0, acc[j]));
                         }
                     }
                 }
