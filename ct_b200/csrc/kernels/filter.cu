@@ -410,10 +410,11 @@ __global__ void __launch_bounds__(1024) filter_kernel(const InT* __restrict__ ra
 // -ln, the weight and the scales), 16 warps per SM and the L1 pipe together: 56 % of
 // the issue slots, 55 % of the L1 wavefronts. 54 instructions per sample; the
 // version before (one row pair per group, scalar operations, twiddles read at a
-// stride) took 84. u16 to FP16, 144 views of 2048^2: 2.11 -> 1.56 ms (1.5 TB/s); 360 of
-// 701 x 409 to FP32 (M = 2048): 1.21 -> 0.64; 360 of 256 x 192 to FP16: 0.104 ->
+// stride) took 84. u16 to FP16, 144 views of 2048^2: 2.11 -> 1.51 ms (1.6 TB/s); 360 of
+// 701 x 409 to FP32 (M = 2048): 1.21 -> 0.60; 360 of 256 x 192 to FP16: 0.104 ->
 // 0.042. Not faster: one code instance for both row pairs (a loop; registers
-// spill: 1.77 ms), five CTAs of 128 threads per SM (102 registers: 1.81).
+// spill: 1.77 ms), five CTAs of 128 threads per SM (102 registers: 1.81), a
+// run-time switch to logf in the whole-number instances (1.66).
 template <int M> struct RF {
     static constexpr int L = M / 16, L2 = L / 16, Q = 16 / L2;
     static constexpr int SA = 16 * (L + L2);       // first transpose, float4 per group
@@ -568,7 +569,7 @@ __device__ __forceinline__ float2 neg_ln2(float2 s) {
 template <int M, bool HALF, typename InT, typename OutT>
 __global__ void __launch_bounds__(RF<M>::T, 512 / RF<M>::T)
     filter_rf_kernel(const InT* __restrict__ raw, OutT* __restrict__ out, FilterArgs a, const float2* __restrict__ tw,
-                     const float* __restrict__ K, int plain_log) {
+                     const float* __restrict__ K) {
     using C = RF<M>;
     constexpr int L = C::L, L2 = C::L2, Q = C::Q, NR = HALF ? 8 : 16;
     const float2* const tw1 = tw + M + threadIdx.x % L;              // pass 1: [s L]
@@ -606,16 +607,16 @@ __global__ void __launch_bounds__(RF<M>::T, 512 / RF<M>::T)
         for (int r = 0; r < NR; ++r)
             p[r] = make_float2(__fmul_rn(raw_value(&x0[r], a), a.log_scale),
                                __fmul_rn(raw_value(&x1[r], a), a.log_scale));
-        // whole-number samples of a positive base intensity are normal and positive; any
-        // other argument (zero, negative, tiny, infinite, NaN) goes to logf
-        bool odd = plain_log;
+        // whole-number samples give normal positive arguments (launch_typed); a float sample
+        // may give any other (zero, negative, tiny, infinite, NaN): those go to logf
+        bool odd = false;
         if constexpr (std::is_same<InT, float>::value) {
 #pragma unroll
             for (int r = 0; r < NR; ++r)
                 odd |= unsigned(__float_as_int(p[r].x) - 0x00800000) >= 0x7f000000u ||
                        unsigned(__float_as_int(p[r].y) - 0x00800000) >= 0x7f000000u;
         }
-        if (__builtin_expect(odd, 0)) {
+        if (std::is_same<InT, float>::value && odd) {
 #pragma unroll
             for (int r = 0; r < NR; ++r) {
                 const float2 c = p[r];
@@ -730,9 +731,7 @@ int launch_rf(const InT* raw, OutT* out, const FilterArgs& a, const float2* tw, 
     const size_t smem = size_t(C::G) * C::SG * sizeof(float4);
     auto kern = filter_rf_kernel<M, HALF, InT, OutT>;
     if (const int st = ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem)) return st;
-    // samples of 8 and 16 bits give arguments from beta to (1 + beta) times the scale
-    const bool normal = a.beta > 0.0f && a.log_scale > 0.0f && a.beta * a.log_scale > 1e-30f && a.log_scale < 1e30f;
-    kern<<<unsigned(blocks), C::T, smem, s>>>(raw, out, a, tw, K, !std::is_same<InT, float>::value && !normal);
+    kern<<<unsigned(blocks), C::T, smem, s>>>(raw, out, a, tw, K);
     return cuda_status(cudaGetLastError(), "filter_rf_kernel launch");
 }
 
@@ -757,7 +756,12 @@ int launch_typed(const InT* raw, OutT* out, const FilterArgs& a, const float2* t
         return CTB_ERR_UNSUPPORTED;
     }
     const bool tab = a.wt != nullptr;
-    if (tab && (a.W == a.M || 2 * a.W <= a.M)) {
+    // the register kernel's logarithm takes normal positive numbers: samples of 8 and 16
+    // bits give arguments from beta to (1 + beta) times the scale, so any but those of a
+    // negative or extreme base intensity; float samples are looked at one by one
+    const bool normal = std::is_same<InT, float>::value || (a.beta > 0.0f && a.log_scale > 0.0f &&
+                                                            a.beta * a.log_scale > 1e-30f && a.log_scale < 1e30f);
+    if (tab && normal && (a.W == a.M || 2 * a.W <= a.M)) {
         switch (a.M) {
             case 256: return launch_rf_any<256>(raw, out, a, tw, K, s);
             case 512: return launch_rf_any<512>(raw, out, a, tw, K, s);

@@ -81,3 +81,21 @@ def test_tiny_samples_match_float64():
     out = ops.filter_projections(torch.from_numpy(raw).cuda(), det, L.RAMLAK, 1, L.FP32).double().cpu().numpy()
     ref = reference(raw, W, 4, 700.0, 1)
     assert np.linalg.norm(out - ref) <= 1e-5 * np.linalg.norm(ref)
+
+
+def test_extreme_base_intensity_takes_the_general_kernel():
+    """A base intensity of 1e-31 puts the logarithm's arguments beyond the register
+    kernel's range for whole-number samples. p is near -71 with a spread of about
+    0.4; half a unit in its last place from the logarithm and from the weight is
+    3e-6, 8e-6 of the spread the ramp keeps: 5e-5 covers it and the transform."""
+    W, H, base = 256, 6, 1e-31
+    rng = np.random.default_rng(3)
+    raw = rng.integers(9000, 60000, (2, H, W)).astype(np.uint16)
+    det, _ = ops.detector(W, H, 700.0, base_intensity=base)
+    out = ops.filter_projections(torch.from_numpy(raw.astype(np.int32)).to(torch.uint16).cuda(), det, L.RAMLAK, 1,
+                                 L.FP32).double().cpu().numpy()
+    u, v = np.arange(W) - W / 2.0, H / 2.0 - np.arange(H)
+    p = -np.log((raw / 65535.0 + 1e-6 * base) / (base + 1e-6 * base))
+    p = p * 700.0 / np.sqrt(700.0 ** 2 + u[None, :] ** 2 + v[:, None] ** 2)
+    ref = np.fft.irfft(np.fft.rfft(p) * (np.arange(W // 2 + 1) / (W // 2 + 1) * W), n=W)
+    assert np.linalg.norm(out - ref) <= 5e-5 * np.linalg.norm(ref)
