@@ -95,10 +95,16 @@ def build(verbose: bool = False, clean: bool = False, checked: bool = True) -> s
             if os.path.isdir(d):
                 shutil.rmtree(d)
     variants = [(False, BUILD, LIB)] + ([(True, CHECKED_BUILD, CHECKED_LIB)] if checked else [])
-    for chk, bdir, lib in variants:
+    for _, bdir, _ in variants:
         os.makedirs(bdir, exist_ok=True)
-        with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as ex:
-            objs = list(ex.map(lambda s: _compile(s, verbose, chk), SOURCES))
+    # every object of both libraries in one pool: the backprojector's file takes
+    # minutes, and the two builds of it run side by side
+    with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as ex:
+        jobs = {chk: [ex.submit(_compile, src, verbose, chk) for src in
+                      sorted(SOURCES, key=lambda f: f != "kernels/backproject_tma.cu")] for chk, _, _ in variants}
+        built = {chk: [j.result() for j in js] for chk, js in jobs.items()}
+    for chk, bdir, lib in variants:
+        objs = built[chk]
         if _newer(lib, objs):
             cmd = [NVCC] + ARCH + ["-shared", "-cudart", "static", "-o", lib] + objs + ["-lz", "-lpthread"]
             if verbose:
