@@ -524,6 +524,12 @@ __device__ __forceinline__ bool tile_pass(const CUtensorMap* map, const T* __res
                     const T* col = proj + (long long)gv * g.view_stride + gu;
                     int ja, jb;
                     v_inside_run(z0, ZC, g.zPre, g.vs, q.z, U, g.lbV, g.ubV, &ja, &jb);
+                    if constexpr (PART) {
+                        // the slab's slices alone: the rows of the tile's other slices (not stored) may lie
+                        // outside a stack that holds only the rows the slab reaches
+                        ja = max(ja, zf);
+                        jb = min(jb, zl - 1);
+                    }
 #pragma unroll
                     for (int j = 0; j < ZC; ++j) {
                         const float vi = row_j(j);
@@ -531,7 +537,8 @@ __device__ __forceinline__ bool tile_pass(const CUtensorMap* map, const T* __res
                             int v0 = int(vi);
                             const float fv = __fsub_rn(vi, float(v0));
 #ifdef CTB_BOUNDS_CHECK
-                            if (!CTB_FETCH_OK(v0, g.H - 1, 4)) v0 = 0;
+                            // (of the rows the stack holds)
+                            if (!CTB_FETCH_OK(v0 - g.row0, (g.rows > 0 ? g.rows : g.H) - 1, 4)) v0 = g.row0;
 #endif
                             const T* r0 = col + (long long)v0 * g.pitch;
                             const float p00 = gval(r0), p01 = gval(r0 + 1);
