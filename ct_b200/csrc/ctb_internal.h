@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <cstddef>
 #include <cstdint>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -102,8 +103,12 @@ struct FilterArgs {
 int build_weight_table(const FilterArgs& a, float* t, cudaStream_t s);
 // Process-wide cache of weight tables per device and geometry. With build = 0
 // (inside a stream capture) only an existing table is returned; a missing one
-// stays null and the filter evaluates the weight per pixel.
-int pre_tables(FilterArgs* a, cudaStream_t s, bool build);
+// stays null and the filter evaluates the weight per pixel. The table is not freed
+// while *pin is held: until the launch that reads it, or as long as a launch may be
+// repeated.
+int pre_tables(FilterArgs* a, cudaStream_t s, bool build, std::shared_ptr<const void>* pin);
+// Hold a pin as long as the graph being captured, and graphs instantiated from it, exist.
+bool keep_for_graph(cudaGraph_t graph, const std::shared_ptr<const void>& pin);
 
 // Launch the fused load/log/weight/FFT/window/IFFT/store kernel over n_views.
 int filter_launch(const void* raw, int raw_type, void* out, int store_type, const FilterArgs& a,

@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <memory>
 #include <new>
 #include <string>
 #include <vector>
@@ -21,6 +22,7 @@ struct ctb_batch {
     std::vector<float4*> views;      // per scan view tables
     std::vector<int> pitch;
     std::vector<ctb::FilterTables> tables;
+    std::vector<std::shared_ptr<const void>> weights;   // pins of the weight tables
     std::vector<ctb::BpBatchScan> bp;
     ctb::BpBatchPlan plan;
     void* d_desc = nullptr;
@@ -159,8 +161,10 @@ int ctb_batch_create(ctb_batch** out, int n, const ctb_scan* scans, int store_ty
         if (st != CTB_OK) return bail(st);
         b->tables.push_back(t);
         // preprocessing tables now: the filters are captured into a graph later
+        // (held, so that a later scan's table does not displace them before the capture)
         FilterArgs pa = filter_args(sc.det, sc.raw_type, t.M, t.logM, sc.n_views, 1.0f);
-        st = pre_tables(&pa, s, true);
+        b->weights.emplace_back();
+        st = pre_tables(&pa, s, true, &b->weights.back());
         if (st != CTB_OK) return bail(st);
         // view table (FP64 geometry kernel)
         float4* v = nullptr;

@@ -863,11 +863,15 @@ int build_weight_table(const FilterArgs& a, float* t, cudaStream_t s) {
 int filter_launch(const void* raw, int raw_type, void* out, int store_type, const FilterArgs& args,
                   const float2* tw, const float* K, cudaStream_t s) {
     FilterArgs a = args;
+    std::shared_ptr<const void> pin;   // the weight table stays until the kernel is launched
     if (!a.wt) {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) cudaGetLastError();
-        const int st = pre_tables(&a, s, cs == cudaStreamCaptureStatusNone);
+        cudaGraph_t graph = nullptr;
+        if (cudaStreamGetCaptureInfo(s, &cs, nullptr, &graph) != cudaSuccess) cudaGetLastError();
+        const int st = pre_tables(&a, s, cs == cudaStreamCaptureStatusNone, &pin);
         if (st != CTB_OK) return st;
+        // a graph reads the table at every launch
+        if (graph && a.wt && !keep_for_graph(graph, pin)) a.wt = nullptr;
     }
     switch (raw_type) {
         case CTB_U8: return launch_out((const uint8_t*)raw, out, store_type, a, tw, K, s);
