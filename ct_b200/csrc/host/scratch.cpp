@@ -15,34 +15,64 @@
 #include <cstdint>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 #include "../ctb_internal.h"
 
 namespace ctb {
 
-unsigned long long current_context_id() {
-    using GetCurrent = CUresult (*)(CUcontext*);
-    using GetId = CUresult (*)(CUcontext, unsigned long long*);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
+namespace {
+// the driver's functions that the runtime has no counterpart of, null when not found
+struct Driver {
+    CUresult (*get_current)(CUcontext*) = nullptr;
+    CUresult (*get_id)(CUcontext, unsigned long long*) = nullptr;
+    CUresult (*primary_state)(CUdevice, unsigned*, int*) = nullptr;
+    CUresult (*primary_retain)(CUcontext*, CUdevice) = nullptr;
+    CUresult (*primary_release)(CUdevice) = nullptr;
+};
+const Driver& driver() {
+    static Driver d;
     static std::once_flag once;
     std::call_once(once, [] {
-        void* a = nullptr;
-        void* b = nullptr;
-        cudaDriverEntryPointQueryResult qa, qb;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &a, cudaEnableDefault, &qa) == cudaSuccess &&
-            qa == cudaDriverEntryPointSuccess &&
-            cudaGetDriverEntryPoint("cuCtxGetId", &b, cudaEnableDefault, &qb) == cudaSuccess &&
-            qb == cudaDriverEntryPointSuccess) {
-            get_current = reinterpret_cast<GetCurrent>(a);
-            get_id = reinterpret_cast<GetId>(b);
-        } else {
-            cudaGetLastError();
-        }
+        auto entry = [](const char* name, auto* fn) {
+            void* p = nullptr;
+            cudaDriverEntryPointQueryResult q;
+            if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess &&
+                q == cudaDriverEntryPointSuccess)
+                *fn = reinterpret_cast<std::remove_pointer_t<decltype(fn)>>(p);
+            else
+                cudaGetLastError();
+        };
+        entry("cuCtxGetCurrent", &d.get_current);
+        entry("cuCtxGetId", &d.get_id);
+        entry("cuDevicePrimaryCtxGetState", &d.primary_state);
+        entry("cuDevicePrimaryCtxRetain", &d.primary_retain);
+        entry("cuDevicePrimaryCtxRelease", &d.primary_release);
     });
+    return d;
+}
+
+// Whether the current context is the device's primary one (the one the CUDA runtime uses).
+bool primary_context_current(int dev) {
+    const Driver& d = driver();
+    CUcontext cur = nullptr, primary = nullptr;
+    unsigned flags = 0;
+    int active = 0;
+    if (!d.get_current || !d.primary_state || !d.primary_retain || !d.primary_release) return false;
+    if (d.get_current(&cur) != CUDA_SUCCESS || d.primary_state(dev, &flags, &active) != CUDA_SUCCESS || !active)
+        return false;
+    if (d.primary_retain(&primary, dev) != CUDA_SUCCESS) return false;
+    d.primary_release(dev);
+    return cur == primary;
+}
+}  // namespace
+
+unsigned long long current_context_id() {
+    const Driver& d = driver();
     CUcontext c = nullptr;
     unsigned long long id = 0;
-    if (!get_current || get_current(&c) != CUDA_SUCCESS || !c || get_id(c, &id) != CUDA_SUCCESS) return 0;
+    if (!d.get_current || !d.get_id || d.get_current(&c) != CUDA_SUCCESS || !c || d.get_id(c, &id) != CUDA_SUCCESS)
+        return 0;
     return id;
 }
 
@@ -57,8 +87,10 @@ struct Pool {
 std::mutex g_pool_mtx;
 std::map<int, Pool> g_pools;
 
-// The current device's pool (null: none to be had, or a capturing stream, whose
-// allocations belong to its graph).
+// The current device's pool (null: none to be had, a capturing stream, whose
+// allocations belong to its graph, or a context beside the device's primary one,
+// where the device's default pool serves: a device has one pool of this library,
+// however many contexts a program switches between).
 cudaMemPool_t scratch_pool(cudaStream_t s) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
@@ -75,6 +107,7 @@ cudaMemPool_t scratch_pool(cudaStream_t s) {
     std::lock_guard<std::mutex> lk(g_pool_mtx);
     Pool& p = g_pools[dev];
     if (p.pool && p.ctx == ctx) return p.pool;
+    if (!primary_context_current(dev)) return nullptr;
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -86,7 +119,7 @@ cudaMemPool_t scratch_pool(cudaStream_t s) {
         return nullptr;
     }
     if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) cudaGetLastError();
-    p.pool = pool;   // (a pool of a context that is gone went with it)
+    p.pool = pool;   // (the pool of a primary context that was reset went with it)
     p.ctx = ctx;
     return pool;
 }
