@@ -16,6 +16,7 @@ const std::string& global_error() { return g_last_error; }
 
 int cuda_status(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return CTB_OK;
+    cudaGetLastError();   // (reported here: the check of a later launch must not find it again)
     g_last_error = std::string(what) + ": " + cudaGetErrorString(e);
     if (e == cudaErrorMemoryAllocation) return CTB_ERR_ALLOC;
     return CTB_ERR_CUDA;
