@@ -65,6 +65,15 @@ int ctb_free_memory(int device, size_t* free_bytes, size_t* total_bytes) {
     return CTB_OK;
 }
 
+int ctb_release_scratch(int device) {
+    int cur = 0;
+    CTB_CUDA_TRY(cudaGetDevice(&cur));
+    CTB_CUDA_TRY(cudaSetDevice(device));
+    ctb::scratch_trim();
+    cudaSetDevice(cur);
+    return CTB_OK;
+}
+
 int ctb_reference_grid(ctb_detector* det, const float rel6[6], ctb_grid* grid) {
     if (!det || !grid || det->width <= 1 || det->height <= 1) return arg_error("invalid detector");
     float r[6] = {0, 1, 0, 1, 0, 1};

@@ -107,6 +107,11 @@ def forward_project(vol, angles_deg, heights_px, det: L.Detector, grid: L.Grid, 
     return out
 
 
+def release_scratch(device=0):
+    """Give the device memory that the operators keep between calls back to the driver."""
+    check(lib().ctb_release_scratch(int(device)))
+
+
 def convert_layout(src, index_order, byte_order=L.LITTLE_ENDIAN, out=None, stream=None):
     """X-fastest slab (Zs, Y, X) -> same bytes in index_order / byte_order (returned as int32 view if swapped)."""
     torch = _torch()

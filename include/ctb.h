@@ -93,6 +93,17 @@ int ctb_device_count(int* count);
 int ctb_device_name(int device, char* buf, size_t buf_len);
 int ctb_free_memory(int device, size_t* free_bytes, size_t* total_bytes);
 
+/* Give the device memory that the operator calls keep back to the driver. A call
+ * takes scratch memory on its stream: 16 bytes per view, ctb_forward_project a
+ * copy of the volume slab, ctb_backproject at rows off 16 bytes a copy of the rows
+ * of a run of views (at most 256 MB, or the bytes of the slab if that is more; it
+ * gathers from the caller's rows if there is no memory for them). Up to 256 MB
+ * of it per device stay with the library for the next call, where other
+ * allocations of the process find it when memory is short; other processes, and
+ * ctb_free_memory, do not see it as free. Memory of calls that are still running
+ * stays with them. No reference counterpart. */
+int ctb_release_scratch(int device);
+
 /* Reference grid for a detector (grid rule Ct/CtVolume.cpp:311-316 and
  * cylinder radius :370-373) with relative bounds rel6 = {xmin,xmax,ymin,ymax,
  * zmin,zmax} clamped like setVolumeBounds (:487-500). det->radius is set. */
