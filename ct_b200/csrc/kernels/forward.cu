@@ -36,8 +36,8 @@
 // reference's v run where the detector's outer rows can tell) is moved inside
 // them, where its other slices weigh 0. Columns with fewer slices than a window,
 // and every column when the volume holds an infinity or NaN (whose product with
-// a zero weight must not reach rows the slice does not touch), take the checked
-// sum instead: each slice weighted by its own v0 and fv.
+// a zero weight must not reach rows the slice does not touch) or a value over
+// 2^100, take the checked sum instead: each slice weighted by its own v0 and fv.
 //
 // What bounds it: the FP32 pipe (an FP32x2 instruction takes two of its cycles):
 // per row and voxel column seven operations for each slice of the window and five
@@ -112,11 +112,15 @@ __device__ __forceinline__ float2 window_sum(const float* __restrict__ p0, const
     return s;
 }
 
-// Row r's sum over the box slices za .. zb of a column among the K from z on:
-// each with the weight of its own v0 and fv, as the backprojector reads it.
-__device__ __forceinline__ float checked_sum(const float* __restrict__ col, float z, int K, int za, int zb, float mdv,
-                                             float c0, int r) {
-    float s = 0.0f;
+// Row r's sums over the box slices za .. zb of a column among the K from z on, for
+// detector columns u0 and u0 + 1: each slice with the weight of its own v0 and fv, as
+// the backprojector reads it. SCALE: of every slice's value times wa and wb (values
+// near the largest float: their sum may be infinite where the products' is not),
+// else both of the value.
+template <bool SCALE>
+__device__ __forceinline__ float2 checked_sum(const float* __restrict__ col, float z, int K, int za, int zb, float mdv,
+                                              float c0, int r, float wa, float wb) {
+    float2 s = make_float2(0.0f, 0.0f);
     const RowLine rl{mdv, c0};
     const int z0 = int(ceilf(fminf(fmaxf(z, -1.0e6f), 1.0e6f)));
     const int z1 = min(z0 + K - 1, zb);
@@ -125,10 +129,12 @@ __device__ __forceinline__ float checked_sum(const float* __restrict__ col, floa
         const int v0 = int(vi);
         const float fv = __fsub_rn(vi, float(v0));
         const float x = __ldg(col + k);
-        if (r == v0) s = fmaf(1.0f - fv, x, s);
-        if (r == v0 + 1) s = fmaf(fv, x, s);
+        if (r != v0 && r != v0 + 1) continue;
+        const float f = r == v0 ? 1.0f - fv : fv;
+        if constexpr (SCALE) s = make_float2(fmaf(f, wa * x, s.x), fmaf(f, wb * x, s.y));
+        else s.x = fmaf(f, x, s.x);
     }
-    return s;
+    return SCALE ? s : make_float2(s.x, s.x);
 }
 
 // Shared memory of a warp: the records of one step, and the sums of the strip's
@@ -183,7 +189,7 @@ __device__ __forceinline__ void hit_rows(const Hit* __restrict__ hits, unsigned 
 }
 
 __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restrict__ volz,
-                                                            const int* __restrict__ nonfinite,
+                                                            const int* __restrict__ extreme,
                                                             const float4* __restrict__ views, ProjGeom g,
                                                             float* __restrict__ proj, int accumulate) {
     constexpr int J = kJ, SW = kSW;
@@ -223,7 +229,7 @@ __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restr
         line_of(double(cs0 + SW) - double(g.uPre), &a1, &b1);
     }
     const float margin = 0.05f + 1.0e-6f * (float(np + ns) + 4.0f * (float(g.W) + fabsf(g.uOff)) / g.vs);
-    const bool all_checked = *nonfinite != 0;
+    const bool all_checked = *extreme != 0;
     const bool edge = all_checked || R <= 1 || R + kRows - 1 >= g.H - 3;   // rows the detector's bounds can cut
     const float r0 = float(R + lane);   // the lane's first row
 #pragma unroll
@@ -316,12 +322,19 @@ __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restr
                         const Hit t = sh.hits[src];
 #pragma unroll
                         for (int j = 0; j < J; ++j) {
-                            const float x = checked_sum(t.line + kMagicBits, fmaf(-(r0 + 32.0f * j), t.inv, t.za), K, a, b,
-                                                        t.mdv, t.c0, R + lane + 32 * j);
+                            const float z = fmaf(-(r0 + 32.0f * j), t.inv, t.za);
+                            const int r = R + lane + 32 * j;
                             float& xa = j & 1 ? ga[j / 2].y : ga[j / 2].x;
                             float& xb = j & 1 ? gb[j / 2].y : gb[j / 2].x;
-                            xa = fmaf(t.wa, x, xa);
-                            xb = fmaf(t.wb, x, xb);
+                            if (all_checked) {
+                                const float2 x = checked_sum<true>(t.line + kMagicBits, z, K, a, b, t.mdv, t.c0, r, t.wa, t.wb);
+                                xa += x.x;
+                                xb += x.y;
+                            } else {
+                                const float2 x = checked_sum<false>(t.line + kMagicBits, z, K, a, b, t.mdv, t.c0, r, 1.0f, 1.0f);
+                                xa = fmaf(t.wa, x.x, xa);
+                                xb = fmaf(t.wb, x.y, xb);
+                            }
                         }
                     }
                 } else {
@@ -365,9 +378,10 @@ __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restr
 }
 
 // z-fastest copy of the slab, [x][y][z], through 32 x 32 shared-memory tiles;
-// *nonfinite is set when a value is infinite or NaN.
+// *extreme is set when a value is NaN or of a magnitude over 2^100: infinite, or one
+// whose sums may be.
 __global__ void volz_kernel(const float* __restrict__ in, int X, int Y, int Zs, float* __restrict__ out,
-                            int* __restrict__ nonfinite) {
+                            int* __restrict__ extreme) {
     __shared__ float tile[32][33];
     const int xt = blockIdx.x * 32, zt = blockIdx.z * 32, y = blockIdx.y;
     const long long plane = (long long)X * Y;
@@ -376,11 +390,11 @@ __global__ void volz_kernel(const float* __restrict__ in, int X, int Y, int Zs, 
         const int z = zt + j, x = xt + threadIdx.x;
         if (z < Zs && x < X) {
             const float v = in[(long long)z * plane + (long long)y * X + x];
-            bad |= !(fabsf(v) <= 3.402823466e38f);
+            bad |= !(fabsf(v) <= 1.2676506e30f);
             tile[j][threadIdx.x] = v;
         }
     }
-    if (bad) *nonfinite = 1;
+    if (bad) *extreme = 1;
     __syncthreads();
     for (int j = threadIdx.y; j < 32; j += 8) {
         const int x = xt + j, z = zt + threadIdx.x;
@@ -405,17 +419,17 @@ int forward_launch(const float* vol, const float4* views, int n_views, const Pro
     const size_t n = size_t(g.X) * g.Y * g.Zs;
     char* scratch = nullptr;
     CTB_CUDA_TRY(scratch_alloc((void**)&scratch, 256 + sizeof(float) * n, s));
-    int* nonfinite = reinterpret_cast<int*>(scratch);
+    int* extreme = reinterpret_cast<int*>(scratch);
     float* volz = reinterpret_cast<float*>(scratch + 256);
-    int st = cuda_status(cudaMemsetAsync(nonfinite, 0, sizeof(int), s), "forward projector flag");
+    int st = cuda_status(cudaMemsetAsync(extreme, 0, sizeof(int), s), "forward projector flag");
     if (st == CTB_OK) {
         volz_kernel<<<dim3((g.X + 31) / 32, g.Y, (g.Zs + 31) / 32), dim3(32, 8), 0, s>>>(vol, g.X, g.Y, g.Zs, volz,
-                                                                                         nonfinite);
+                                                                                         extreme);
         st = cuda_status(cudaGetLastError(), "volz_kernel launch");
     }
     if (st == CTB_OK) {
         const dim3 grid((g.W + kWarps * kSW - 1) / (kWarps * kSW), n_views, (g.H + kRows - 1) / kRows);
-        fp_kernel<<<grid, dim3(32, kWarps), 0, s>>>(volz, nonfinite, views, g, proj, accumulate);
+        fp_kernel<<<grid, dim3(32, kWarps), 0, s>>>(volz, extreme, views, g, proj, accumulate);
         st = cuda_status(cudaGetLastError(), "fp_kernel launch");
     }
     cudaFreeAsync(scratch, s);
