@@ -34,10 +34,12 @@
 //     strip's sums in shared memory between groups.
 // A window that would leave the slices that count (the slab, cut to the
 // reference's v run where the detector's outer rows can tell) is moved inside
-// them, where its other slices weigh 0. Columns with fewer slices than a window,
-// and every column when the volume holds an infinity or NaN (whose product with
-// a zero weight must not reach rows the slice does not touch) or a value over
-// 2^100, take the checked sum instead: each slice weighted by its own v0 and fv.
+// them, where its other slices weigh 0; a volume that holds an infinity or NaN (whose
+// product with a zero weight must not reach rows the slice does not touch) or a value
+// over 2^100 is summed slice by slice, those that do not touch a row left out.
+// Elsewhere columns with fewer slices than a window take a checked sum: each slice
+// weighted by its own v0 and fv (128^3 with one NaN, 120 views of 256 x 192: 1.32 ms;
+// by checked sums throughout 1.64, the slice walk of the version before 1.41).
 //
 // What bounds it: the FP32 pipe (an FP32x2 instruction takes two of its cycles):
 // per row and voxel column seven operations for each slice of the window and five
@@ -73,6 +75,7 @@ constexpr unsigned kAll = 0xffffffffu;
 // detector columns and kJ rows per lane
 constexpr int kWarps = 4, kSW = 4, kJ = 4, kRows = 32 * kJ;
 constexpr float kMagic = 12582912.0f;       // 1.5 * 2^23: rounds to an integer by one add
+constexpr int kExtreme = 1 << 22;           // marks a window's length in an extreme volume
 constexpr int kMagicBits = 0x4B400000;      // its bits: the low bits of integer + kMagic are the integer
 
 // One voxel column that reaches a warp's strip and rows.
@@ -84,17 +87,20 @@ struct __align__(16) Hit {
     float wa, wb;       // weight of detector columns u0 and u0 + 1
 };
 
-// d = vi(z) - r and the weights 1 - |d| (0 beyond 1) of two rows' slices z, given
-// as the bits of z + kMagic. vi as row_at forms it, fma(z mod 32, mdv, fma(z - z
-// mod 32, mdv, c0)): the block's start is the integer with its low five bits
-// cleared, z mod 32 the difference of the two floats (exact). The integer steps
-// run beside the FMA pipe, which bounds this kernel.
-__device__ __forceinline__ float2 weights(int zx, int zy, float2 nrf, float2 mdv, float2 c0) {
+// d = vi(z) - r of two rows' slices z, given as the bits of z + kMagic. vi as row_at
+// forms it, fma(z mod 32, mdv, fma(z - z mod 32, mdv, c0)): the block's start is the
+// integer with its low five bits cleared, z mod 32 the difference of the two floats
+// (exact). The integer steps run beside the FMA pipe, which bounds this kernel.
+__device__ __forceinline__ float2 row_distances(int zx, int zy, float2 nrf, float2 mdv, float2 c0) {
     const float2 zm = make_float2(__int_as_float(zx), __int_as_float(zy));
     const float2 bm = make_float2(__int_as_float(zx & ~31), __int_as_float(zy & ~31));
     const float2 zb = __fadd2_rn(bm, make_float2(-kMagic, -kMagic));
     const float2 zo = __ffma2_rn(bm, make_float2(-1.0f, -1.0f), zm);
-    const float2 d = __fadd2_rn(__ffma2_rn(zo, mdv, __ffma2_rn(zb, mdv, c0)), nrf);
+    return __fadd2_rn(__ffma2_rn(zo, mdv, __ffma2_rn(zb, mdv, c0)), nrf);
+}
+// The weights 1 - |d|, 0 beyond 1.
+__device__ __forceinline__ float2 weights(int zx, int zy, float2 nrf, float2 mdv, float2 c0) {
+    const float2 d = row_distances(zx, zy, nrf, mdv, c0);
     return make_float2(__saturatef(1.0f - fabsf(d.x)), __saturatef(1.0f - fabsf(d.y)));
 }
 
@@ -112,15 +118,11 @@ __device__ __forceinline__ float2 window_sum(const float* __restrict__ p0, const
     return s;
 }
 
-// Row r's sums over the box slices za .. zb of a column among the K from z on, for
-// detector columns u0 and u0 + 1: each slice with the weight of its own v0 and fv, as
-// the backprojector reads it. SCALE: of every slice's value times wa and wb (values
-// near the largest float: their sum may be infinite where the products' is not),
-// else both of the value.
-template <bool SCALE>
-__device__ __forceinline__ float2 checked_sum(const float* __restrict__ col, float z, int K, int za, int zb, float mdv,
-                                              float c0, int r, float wa, float wb) {
-    float2 s = make_float2(0.0f, 0.0f);
+// Row r's sum over the box slices za .. zb of a column among the K from z on:
+// each with the weight of its own v0 and fv, as the backprojector reads it.
+__device__ __forceinline__ float checked_sum(const float* __restrict__ col, float z, int K, int za, int zb, float mdv,
+                                             float c0, int r) {
+    float s = 0.0f;
     const RowLine rl{mdv, c0};
     const int z0 = int(ceilf(fminf(fmaxf(z, -1.0e6f), 1.0e6f)));
     const int z1 = min(z0 + K - 1, zb);
@@ -129,12 +131,10 @@ __device__ __forceinline__ float2 checked_sum(const float* __restrict__ col, flo
         const int v0 = int(vi);
         const float fv = __fsub_rn(vi, float(v0));
         const float x = __ldg(col + k);
-        if (r != v0 && r != v0 + 1) continue;
-        const float f = r == v0 ? 1.0f - fv : fv;
-        if constexpr (SCALE) s = make_float2(fmaf(f, wa * x, s.x), fmaf(f, wb * x, s.y));
-        else s.x = fmaf(f, x, s.x);
+        if (r == v0) s = fmaf(1.0f - fv, x, s);
+        if (r == v0 + 1) s = fmaf(fv, x, s);
     }
-    return SCALE ? s : make_float2(s.x, s.x);
+    return s;
 }
 
 // Shared memory of a warp: the records of one step, and the sums of the strip's
@@ -147,8 +147,10 @@ struct WarpShared {
 
 // The rows of the hit columns `same` (lanes' records), all with windows of K
 // slices (KC, or K at run time for KC = 0): gives their sums times w (1-fu) and
-// w fu. r0: the lane's first row.
-template <int JU, int KC>
+// w fu. r0: the lane's first row. EXTREME: the volume holds an infinity, a NaN or
+// values near the largest float: slices that do not count or do not touch a row are
+// left out (not taken times 0), and values are weighted before they are summed.
+template <int JU, int KC, bool EXTREME = false>
 __device__ __forceinline__ void hit_rows(const Hit* __restrict__ hits, unsigned same, int K, float r0,
                                          float2 (&ga)[kJ / 2], float2 (&gb)[kJ / 2]) {
 #pragma unroll
@@ -166,6 +168,33 @@ __device__ __forceinline__ void hit_rows(const Hit* __restrict__ hits, unsigned 
 #pragma unroll
         for (int i = 0; i < JU / 2; ++i) {
             float2 z = make_float2(fmaf(-64.0f * i, t.inv, za), fmaf(-64.0f * i - 32.0f, t.inv, za));
+            if constexpr (EXTREME) {
+                // slices zmin .. zb count (the window may lie beyond them)
+                const float zb = t.zmax + float(K - 1);
+                z = make_float2(fminf(fmaxf(z.x, t.zmin - float(K)), zb + 1.0f),
+                                fminf(fmaxf(z.y, t.zmin - float(K)), zb + 1.0f));
+                const float2 zm = __fadd2_ru(z, make_float2(kMagic, kMagic));   // ceil
+                const int za = kMagicBits + int(t.zmin), ze = kMagicBits + int(zb);
+                const int sx = __float_as_int(zm.x), sy = __float_as_int(zm.y);
+                const int k1 = min(K - 1, ze - min(sx, sy));
+                for (int k = max(0, za - max(sx, sy)); k <= k1; ++k) {
+                    const int zx = sx + k, zy = sy + k;
+                    const float2 d = row_distances(zx, zy, nr[i], mdv2, c02);
+                    // (a kept slice's row is 0 at least, as int() makes it)
+                    const float dx = fmaxf(d.x, nr[i].x), dy = fmaxf(d.y, nr[i].y);
+                    if (zx >= za && zx <= ze && dx >= -1.0f && dx < 1.0f) {   // r is v0 or v0 + 1
+                        const float v = __ldg(t.line + zx);
+                        ga[i].x = fmaf(1.0f - fabsf(dx), t.wa * v, ga[i].x);
+                        gb[i].x = fmaf(1.0f - fabsf(dx), t.wb * v, gb[i].x);
+                    }
+                    if (zy >= za && zy <= ze && dy >= -1.0f && dy < 1.0f) {
+                        const float v = __ldg(t.line + zy);
+                        ga[i].y = fmaf(1.0f - fabsf(dy), t.wa * v, ga[i].y);
+                        gb[i].y = fmaf(1.0f - fabsf(dy), t.wb * v, gb[i].y);
+                    }
+                }
+                continue;
+            }
             // a window stays inside the slices that count: one moved there has only
             // weights of 0 but for the slices it shares with the one it stands for
             z = make_float2(fminf(fmaxf(z.x, t.zmin), t.zmax), fminf(fmaxf(z.y, t.zmin), t.zmax));
@@ -189,7 +218,7 @@ __device__ __forceinline__ void hit_rows(const Hit* __restrict__ hits, unsigned 
 }
 
 __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restrict__ volz,
-                                                            const int* __restrict__ extreme,
+                                                            const int* __restrict__ extreme_flag,
                                                             const float4* __restrict__ views, ProjGeom g,
                                                             float* __restrict__ proj, int accumulate) {
     constexpr int J = kJ, SW = kSW;
@@ -229,8 +258,8 @@ __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restr
         line_of(double(cs0 + SW) - double(g.uPre), &a1, &b1);
     }
     const float margin = 0.05f + 1.0e-6f * (float(np + ns) + 4.0f * (float(g.W) + fabsf(g.uOff)) / g.vs);
-    const bool all_checked = *extreme != 0;
-    const bool edge = all_checked || R <= 1 || R + kRows - 1 >= g.H - 3;   // rows the detector's bounds can cut
+    const int extreme = *extreme_flag != 0 ? kExtreme : 0;
+    const bool edge = R <= 1 || R + kRows - 1 >= g.H - 3;   // rows the detector's bounds can cut
     const float r0 = float(R + lane);   // the lane's first row
 #pragma unroll
     for (int k = 0; k < SW + 2; ++k)
@@ -285,7 +314,7 @@ __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restr
                         if (hit && edge && !(vb >= 0.5f && vt <= g.vi_hi - 0.5f))
                             v_inside_run(0, g.Zs, g.zPre, g.vs, h, U, g.lbV, g.ubV, &ja, &jb);
                         hit = hit && ja <= jb;
-                        const bool check = all_checked || jb - ja + 1 < K ||
+                        const bool check = jb - ja + 1 < K ||
                                            (edge && vb < 0.5f && row_at(rl, g.z_begin + jb) < 0.0f);
                         if (hit) {
                             what = (u0 - cs0 + 1) | int(check) << 7 | K << 8;
@@ -311,9 +340,9 @@ __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restr
                 const int lead = __shfl_sync(kAll, what, __ffs(mask) - 1);
                 const unsigned same = __ballot_sync(kAll, what == lead);
                 mask &= ~same;
-                const int K = lead >> 8;
+                const int K = lead >> 8 | extreme;
                 float2 ga[J / 2], gb[J / 2];
-                if (lead & 128) {
+                if ((lead & 128) && !extreme) {
 #pragma unroll
                     for (int i = 0; i < J / 2; ++i) ga[i] = gb[i] = make_float2(0.0f, 0.0f);
                     for (unsigned e = same; e; e &= e - 1) {
@@ -322,19 +351,12 @@ __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restr
                         const Hit t = sh.hits[src];
 #pragma unroll
                         for (int j = 0; j < J; ++j) {
-                            const float z = fmaf(-(r0 + 32.0f * j), t.inv, t.za);
-                            const int r = R + lane + 32 * j;
+                            const float x = checked_sum(t.line + kMagicBits, fmaf(-(r0 + 32.0f * j), t.inv, t.za), K, a, b,
+                                                        t.mdv, t.c0, R + lane + 32 * j);
                             float& xa = j & 1 ? ga[j / 2].y : ga[j / 2].x;
                             float& xb = j & 1 ? gb[j / 2].y : gb[j / 2].x;
-                            if (all_checked) {
-                                const float2 x = checked_sum<true>(t.line + kMagicBits, z, K, a, b, t.mdv, t.c0, r, t.wa, t.wb);
-                                xa += x.x;
-                                xb += x.y;
-                            } else {
-                                const float2 x = checked_sum<false>(t.line + kMagicBits, z, K, a, b, t.mdv, t.c0, r, 1.0f, 1.0f);
-                                xa = fmaf(t.wa, x.x, xa);
-                                xb = fmaf(t.wb, x.y, xb);
-                            }
+                            xa = fmaf(t.wa, x, xa);
+                            xb = fmaf(t.wb, x, xb);
                         }
                     }
                 } else {
@@ -345,7 +367,10 @@ __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restr
                             case 2: hit_rows<JU, 2>(sh.hits, same, K, r0, ga, gb); break;
                             case 3: hit_rows<JU, 3>(sh.hits, same, K, r0, ga, gb); break;
                             case 4: hit_rows<JU, 4>(sh.hits, same, K, r0, ga, gb); break;
-                            default: hit_rows<JU, 0>(sh.hits, same, K, r0, ga, gb); break;
+                            default:
+                                if (K & kExtreme) hit_rows<JU, 0, true>(sh.hits, same, K & ~kExtreme, r0, ga, gb);
+                                else hit_rows<JU, 0>(sh.hits, same, K, r0, ga, gb);
+                                break;
                         }
                     };
                     // (a last row block with 64 rows or fewer skips the others)
