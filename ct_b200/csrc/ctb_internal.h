@@ -163,7 +163,7 @@ void slab_row_band(const ProjGeom& g, double hlo, double hhi, int* r_lo, int* ro
 // Backprojection of views [0, n) from `views` (device view table) into vol.
 // hmax bounds |height offset| (pixels) over the views. Dispatches to the
 // shared-memory (TMA) kernel when possible, else to the global-gather kernel.
-int bp_pick_zc(int slab_slices);
+int bp_pick_zc(int z_begin, int slab_slices);
 // Launch shape of the shared-memory backprojector; 0 = the built-in choice.
 struct BpConfig {
     int zc = 0;     // z voxels per thread (8, 16 or 32): the block tile's height
@@ -179,11 +179,11 @@ int backproject_global_launch(const void* proj, int store_type, const float4* vi
 // does not suit the TMA kernel. zc: z voxels per thread (8, 16 or 32).
 int backproject_tma_launch(const void* proj, int store_type, const float4* views, int n_views,
                            const ProjGeom& g, double hmax, float* vol, int accumulate, cudaStream_t s,
-                           int zc = 16, int nbuf = 0);
+                           int zc = 16, int nbuf = 0, int ctas = 1);
 // Whether the TMA kernel takes this layout (16-byte base and strides), and
-// whether its boxes fit this geometry.
+// whether its boxes fit this geometry with `ctas` CTAs on an SM.
 bool backproject_tma_layout(const void* proj, int store_type, const ProjGeom& g);
-bool backproject_tma_fits(int store_type, const ProjGeom& g, double hmax, int zc, int nbuf);
+bool backproject_tma_fits(int store_type, const ProjGeom& g, double hmax, int zc, int nbuf, int ctas);
 // Copy rows row0 .. row0 + rows - 1 of n views (row pitch src_pitch, views
 // src_stride apart, any alignment of the element type) to dst, dense with
 // row pitch dst_pitch (a multiple of 16 bytes, dst 16-byte aligned).

@@ -235,13 +235,28 @@ ProjGeom proj_geom(const ctb_detector& det, const ctb_grid& grid, int z_begin, i
     return g;
 }
 
-// z voxels per thread of the shared-memory backprojector: 32 spreads each
-// column's per-view geometry over twice the voxels of 16 (8% faster on the
-// 128-slice slabs of a 1024^3 volume, with 3 instead of 4 CTAs per SM; 64
-// at 2 CTAs per SM was slower again). The slices of a slab's last tile that lie
-// past it cost little (a tile skips them in groups of eight), so slabs take the
-// smallest tile that holds 32, 16 or 8 slices.
-int bp_pick_zc(int Zs) { return Zs > 16 ? 32 : Zs > 8 ? 16 : 8; }
+// z voxels per thread of the shared-memory backprojector: 32 spreads each column's
+// per-view geometry over twice the voxels of 16 (8 % faster on the 128-slice slabs of
+// a 1024^3 volume, with 3 instead of 4 CTAs per SM; 64 at 2 CTAs per SM was slower
+// again), but a tile is summed whole, or group of eight by group of eight where it
+// holds half its slices or fewer, which costs more per slice. Of 32 and 16 the
+// one whose tiles take less time: 600 x 600 columns of 1.3 pixels, 60 views of 1024 x 512,
+// ms a layer of tiles, FP32 / FP16: 32 whole 0.45 / 0.51, two groups 0.35 / 0.39, one 0.23 / 0.26; 16
+// whole 0.26 / 0.29, one group 0.20 / 0.21. Slices 0 .. 40 0.82 in tiles of 32, 0.79 in tiles of
+// 16; 16 .. 47 0.75 and 0.54; 0 .. 79 1.24 and 1.28. Up to 16 slices take 16 or 8.
+int bp_pick_zc(int z_begin, int Zs) {
+    if (Zs <= 16) return Zs > 8 ? 16 : 8;
+    const int cost32[5] = {0, 8, 12, 16, 16}, cost16[3] = {0, 7, 9};   // by groups of eight in the slab
+    auto cost = [&](int zc, const int* per_tile) {
+        long long c = 0;
+        for (int z = z_begin / zc * zc; z < z_begin + Zs; z += zc) {
+            const int first = std::max(z, z_begin) / 8, last = (std::min(z + zc, z_begin + Zs) - 1) / 8;
+            c += per_tile[last - first + 1];
+        }
+        return c;
+    };
+    return cost(16, cost16) <= cost(32, cost32) ? 16 : 32;
+}
 
 namespace {
 
@@ -366,10 +381,15 @@ int backproject_launch(const void* proj, int store_type, const float4* views, in
         return (v == 8 || v == 16 || v == 32) ? v : 0;
     }();
     if (variant != 1) {
-        const int zc = zc_env ? zc_env : cfg.zc ? cfg.zc : bp_pick_zc(g.Zs);
+        const int zc = zc_env ? zc_env : cfg.zc ? cfg.zc : bp_pick_zc(g.z_begin, g.Zs);
+        // tiles of 32 need two CTAs on an SM, or 16 is taken: voxels of 4 pixels FP32, whose boxes
+        // leave one, 256 x 256 x 64 from 60 views of 1024 x 768 0.33 ms, tiles of 16 0.26; of 3.5 pixels (two
+        // CTAs) 0.225 and 0.246
+        const int ctas = zc == 32 && !zc_env && !cfg.zc ? 2 : 1;
         int st = CTB_ERR_UNSUPPORTED;
         if (backproject_tma_layout(proj, store_type, g)) {
-            st = backproject_tma_launch(proj, store_type, views, n_views, g, hmax, vol, accumulate, s, zc, cfg.nbuf);
+            st = backproject_tma_launch(proj, store_type, views, n_views, g, hmax, vol, accumulate, s, zc, cfg.nbuf,
+                                        ctas);
             // a taller tile's footprint may exceed the box limits where a shorter one fits
             if (st == CTB_ERR_UNSUPPORTED && !zc_env && zc > 16)
                 st = backproject_tma_launch(proj, store_type, views, n_views, g, hmax, vol, accumulate, s, 16);
@@ -384,10 +404,10 @@ int backproject_launch(const void* proj, int store_type, const float4* views, in
             slab_row_band(g, -hmax, hmax, &lo, &rows);
             const double updates = double(g.X) * g.Y * g.Zs, samples = double(g.W) * rows;
             if (2.0 * updates >= samples) {
-                if (backproject_tma_fits(store_type, g, hmax, zc, cfg.nbuf))
+                if (backproject_tma_fits(store_type, g, hmax, zc, cfg.nbuf, ctas))
                     st = backproject_repacked(proj, store_type, views, n_views, g, hmax, vol, accumulate, s, zc,
                                               cfg.nbuf);
-                else if (!zc_env && zc > 16 && backproject_tma_fits(store_type, g, hmax, 16, 0))
+                else if (!zc_env && zc > 16 && backproject_tma_fits(store_type, g, hmax, 16, 0, 1))
                     st = backproject_repacked(proj, store_type, views, n_views, g, hmax, vol, accumulate, s, 16, 0);
             }
         }
