@@ -99,6 +99,9 @@ struct FilterArgs {
     const float* wt = nullptr;
 };
 
+// Rows of a weight table: the detector's, twice over for low detectors of 4 k + 2
+// rows, whose views the register filter takes two at a time.
+inline int weight_rows(int H) { return H % 4 == 2 && H < 64 ? 2 * H : H; }
 // Build that table (exactly the per-pixel operations, evaluated once).
 int build_weight_table(const FilterArgs& a, float* t, cudaStream_t s);
 // Process-wide cache of weight tables per device and geometry. With build = 0

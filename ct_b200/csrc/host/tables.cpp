@@ -117,7 +117,7 @@ int pre_tables(FilterArgs* a, cudaStream_t s, bool build, std::shared_ptr<const 
     CTB_CUDA_TRY(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lk(g_mtx);
     const PreKey k{dev, a->W, a->H, bits(a->D), bits(a->uPre), bits(a->vPre)};
-    return pre_table(k, size_t(a->W) * a->H, build, [&](float* t) {
+    return pre_table(k, size_t(a->W) * weight_rows(a->H), build, [&](float* t) {
         int r = build_weight_table(*a, t, s);
         if (r == CTB_OK) r = cuda_status(cudaStreamSynchronize(s), "weight table");
         return r;
