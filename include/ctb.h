@@ -141,7 +141,8 @@ int ctb_filter_projections(const void* raw, int raw_type, int n_views, const ctb
  * Replaces startReconstruction / reconstructionKernel (Ct/cuda_ct.h:47-69,
  * Ct/cuda_ct.cu:201-352), which adds one view per launch into a pitched chunk.
  *   angles_deg / height_offsets_px: host arrays (n_views), after the
- *     reference's direction correction and relative height offsets.
+ *     reference's direction correction and relative height offsets. Read before
+ *     the call returns (a captured graph keeps the values of the capture).
  *   load_scale: multiplies every sample (1/store_scale of the filter).
  *   accumulate: 0 = overwrite the slab, 1 = add to it. */
 int ctb_backproject(const void* filtered, int store_type, int n_views, const double* angles_deg,
@@ -149,11 +150,15 @@ int ctb_backproject(const void* filtered, int store_type, int n_views, const dou
                     int z_begin, int z_end, float load_scale, float* vol, int accumulate, void* stream);
 
 /* ctb_backproject for callers that cannot allocate device memory. No
- * counterpart in the reference. Same arguments and result as ctb_backproject,
- * but the per-view geometry table that ctb_backproject allocates on the stream
- * at every call lives in a static 256 KB device array of the library instead,
- * so this call allocates nothing (the caller passes the filtered projections
- * and the volume, as before). At most CTB_NOALLOC_MAX_VIEWS views per call
+ * counterpart in the reference. Same arguments as ctb_backproject, but the
+ * per-view geometry table that ctb_backproject takes on the stream lives in a
+ * static 256 KB device array of the library instead, and nothing else is taken
+ * (the caller passes the filtered projections and the volume, as before). The
+ * volume is the same, bit for bit, where rows start on 16 bytes: the base pointer,
+ * and a width that is a multiple of 8 (16-bit storage) or 4 (FP32) samples.
+ * Other rows ctb_backproject copies to its scratch memory; this call gathers from
+ * them where they are: the same voxel and row decisions, sums within rounding
+ * (2e-6 relative L2), several times slower. At most CTB_NOALLOC_MAX_VIEWS views per call
  * (CTB_ERR_UNSUPPORTED beyond that); larger sets of views are split into
  * several calls with accumulate = 1. Arguments are checked as ctb_backproject
  * checks them. The first call on a device looks up the array's address, which
