@@ -193,13 +193,14 @@ int ctb_diag_bounds_status(int device, int* checked_build, unsigned* violations,
     int prev = 0;
     CTB_CUDA_TRY(cudaGetDevice(&prev));
     CTB_CUDA_TRY(cudaSetDevice(device));
-    unsigned c1 = 0, c2 = 0;
-    unsigned long long f1 = 0, f2 = 0;
+    unsigned c1 = 0, c2 = 0, c3 = 0;
+    unsigned long long f1 = 0, f2 = 0, f3 = 0;
     int st = ctb::bounds_status_tma(&c1, &f1, reset);
     if (st == CTB_OK) st = ctb::bounds_status_gather(&c2, &f2, reset);
+    if (st == CTB_OK) st = ctb::bounds_status_forward(&c3, &f3, reset);
     cudaSetDevice(prev);
-    *violations = c1 + c2;
-    *first = f1 ? f1 : f2;
+    *violations = c1 + c2 + c3;
+    *first = f1 ? f1 : f2 ? f2 : f3;
     return st;
 }
 

@@ -225,10 +225,11 @@ int bp_batch_launch(const BpBatchPlan& plan, const void* desc, const long long* 
 // exceeds the box do (0 = off). Results do not change.
 void bp_force_overflow(int every);
 // Bounds-checked build: out-of-range texel fetches recorded by the shared-memory
-// (TMA) and global-gather backprojectors since the last reset; always 0 in the
-// normal build.
+// (TMA) and global-gather backprojectors and of the forward projector since the last
+// reset; always 0 in the normal build.
 int bounds_status_tma(unsigned* count, unsigned long long* first, int reset);
 int bounds_status_gather(unsigned* count, unsigned long long* first, int reset);
+int bounds_status_forward(unsigned* count, unsigned long long* first, int reset);
 // Number of CTAs whose bounded mbarrier waits gave up since the last reset.
 int device_wait_timeouts(unsigned* count, int reset);
 // Run a wait that can never complete with the given try limit (diagnostic of

@@ -104,14 +104,23 @@ __device__ __forceinline__ float2 weights(int zx, int zy, float2 nrf, float2 mdv
     return make_float2(__saturatef(1.0f - fabsf(d.x)), __saturatef(1.0f - fabsf(d.y)));
 }
 
+// The volume copy, for the bounds-checked build.
+struct VolRange {
+    const float* p;
+    long long n;
+};
+__device__ __forceinline__ float fetch(const float* q, const VolRange& vol, unsigned site) {
+    return CTB_FETCH_OK(q - vol.p, vol.n, site) ? __ldg(q) : 0.0f;
+}
+
 // Weighted sums over K slices for two rows whose windows start at the slices of
 // bits zx, zy (lines p0, p1 start there).
 template <int K>
 __device__ __forceinline__ float2 window_sum(const float* __restrict__ p0, const float* __restrict__ p1, int zx,
-                                             int zy, float2 nrf, float2 mdv, float2 c0) {
+                                             int zy, float2 nrf, float2 mdv, float2 c0, const VolRange& vol) {
     float2 v[K];
 #pragma unroll
-    for (int k = 0; k < K; ++k) v[k] = make_float2(__ldg(p0 + k), __ldg(p1 + k));
+    for (int k = 0; k < K; ++k) v[k] = make_float2(fetch(p0 + k, vol, 6), fetch(p1 + k, vol, 6));
     float2 s = __fmul2_rn(weights(zx, zy, nrf, mdv, c0), v[0]);
 #pragma unroll
     for (int k = 1; k < K; ++k) s = __ffma2_rn(weights(zx + k, zy + k, nrf, mdv, c0), v[k], s);
@@ -121,7 +130,7 @@ __device__ __forceinline__ float2 window_sum(const float* __restrict__ p0, const
 // Row r's sum over the box slices za .. zb of a column among the K from z on:
 // each with the weight of its own v0 and fv, as the backprojector reads it.
 __device__ __forceinline__ float checked_sum(const float* __restrict__ col, float z, int K, int za, int zb, float mdv,
-                                             float c0, int r) {
+                                             float c0, int r, const VolRange& vol) {
     float s = 0.0f;
     const RowLine rl{mdv, c0};
     const int z0 = int(ceilf(fminf(fmaxf(z, -1.0e6f), 1.0e6f)));
@@ -130,7 +139,7 @@ __device__ __forceinline__ float checked_sum(const float* __restrict__ col, floa
         const float vi = row_at(rl, k);
         const int v0 = int(vi);
         const float fv = __fsub_rn(vi, float(v0));
-        const float x = __ldg(col + k);
+        const float x = fetch(col + k, vol, 7);
         if (r == v0) s = fmaf(1.0f - fv, x, s);
         if (r == v0 + 1) s = fmaf(fv, x, s);
     }
@@ -152,7 +161,7 @@ struct WarpShared {
 // left out (not taken times 0), and values are weighted before they are summed.
 template <int JU, int KC, bool EXTREME = false>
 __device__ __forceinline__ void hit_rows(const Hit* __restrict__ hits, unsigned same, int K, float r0,
-                                         float2 (&ga)[kJ / 2], float2 (&gb)[kJ / 2]) {
+                                         float2 (&ga)[kJ / 2], float2 (&gb)[kJ / 2], const VolRange& vol) {
 #pragma unroll
     for (int i = 0; i < kJ / 2; ++i) ga[i] = gb[i] = make_float2(0.0f, 0.0f);
     float2 nr[JU / 2];   // the lane's rows, negated
@@ -183,12 +192,12 @@ __device__ __forceinline__ void hit_rows(const Hit* __restrict__ hits, unsigned 
                     // (a kept slice's row is 0 at least, as int() makes it)
                     const float dx = fmaxf(d.x, nr[i].x), dy = fmaxf(d.y, nr[i].y);
                     if (zx >= za && zx <= ze && dx >= -1.0f && dx < 1.0f) {   // r is v0 or v0 + 1
-                        const float v = __ldg(t.line + zx);
+                        const float v = fetch(t.line + zx, vol, 8);
                         ga[i].x = fmaf(1.0f - fabsf(dx), t.wa * v, ga[i].x);
                         gb[i].x = fmaf(1.0f - fabsf(dx), t.wb * v, gb[i].x);
                     }
                     if (zy >= za && zy <= ze && dy >= -1.0f && dy < 1.0f) {
-                        const float v = __ldg(t.line + zy);
+                        const float v = fetch(t.line + zy, vol, 8);
                         ga[i].y = fmaf(1.0f - fabsf(dy), t.wa * v, ga[i].y);
                         gb[i].y = fmaf(1.0f - fabsf(dy), t.wb * v, gb[i].y);
                     }
@@ -204,12 +213,12 @@ __device__ __forceinline__ void hit_rows(const Hit* __restrict__ hits, unsigned 
             const float* p1 = t.line + zy;
             float2 s;
             if constexpr (KC > 0) {
-                s = window_sum<KC>(p0, p1, zx, zy, nr[i], mdv2, c02);
+                s = window_sum<KC>(p0, p1, zx, zy, nr[i], mdv2, c02, vol);
             } else {
                 s = make_float2(0.0f, 0.0f);
                 for (int k = 0; k < K; ++k)
                     s = __ffma2_rn(weights(zx + k, zy + k, nr[i], mdv2, c02),
-                                   make_float2(__ldg(p0 + k), __ldg(p1 + k)), s);
+                                   make_float2(fetch(p0 + k, vol, 6), fetch(p1 + k, vol, 6)), s);
             }
             ga[i] = __ffma2_rn(wa2, s, ga[i]);
             gb[i] = __ffma2_rn(wb2, s, gb[i]);
@@ -261,6 +270,7 @@ __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restr
     const int extreme = *extreme_flag != 0 ? kExtreme : 0;
     const bool edge = R <= 1 || R + kRows - 1 >= g.H - 3;   // rows the detector's bounds can cut
     const float r0 = float(R + lane);   // the lane's first row
+    const VolRange vol{volz, (long long)g.X * g.Y * g.Zs};
 #pragma unroll
     for (int k = 0; k < SW + 2; ++k)
 #pragma unroll
@@ -352,7 +362,7 @@ __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restr
 #pragma unroll
                         for (int j = 0; j < J; ++j) {
                             const float x = checked_sum(t.line + kMagicBits, fmaf(-(r0 + 32.0f * j), t.inv, t.za), K, a, b,
-                                                        t.mdv, t.c0, R + lane + 32 * j);
+                                                        t.mdv, t.c0, R + lane + 32 * j, vol);
                             float& xa = j & 1 ? ga[j / 2].y : ga[j / 2].x;
                             float& xb = j & 1 ? gb[j / 2].y : gb[j / 2].x;
                             xa = fmaf(t.wa, x, xa);
@@ -363,13 +373,13 @@ __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restr
                     auto take = [&](auto used) {
                         constexpr int JU = decltype(used)::value;
                         switch (K) {
-                            case 1: hit_rows<JU, 1>(sh.hits, same, K, r0, ga, gb); break;
-                            case 2: hit_rows<JU, 2>(sh.hits, same, K, r0, ga, gb); break;
-                            case 3: hit_rows<JU, 3>(sh.hits, same, K, r0, ga, gb); break;
-                            case 4: hit_rows<JU, 4>(sh.hits, same, K, r0, ga, gb); break;
+                            case 1: hit_rows<JU, 1>(sh.hits, same, K, r0, ga, gb, vol); break;
+                            case 2: hit_rows<JU, 2>(sh.hits, same, K, r0, ga, gb, vol); break;
+                            case 3: hit_rows<JU, 3>(sh.hits, same, K, r0, ga, gb, vol); break;
+                            case 4: hit_rows<JU, 4>(sh.hits, same, K, r0, ga, gb, vol); break;
                             default:
-                                if (K & kExtreme) hit_rows<JU, 0, true>(sh.hits, same, K & ~kExtreme, r0, ga, gb);
-                                else hit_rows<JU, 0>(sh.hits, same, K, r0, ga, gb);
+                                if (K & kExtreme) hit_rows<JU, 0, true>(sh.hits, same, K & ~kExtreme, r0, ga, gb, vol);
+                                else hit_rows<JU, 0>(sh.hits, same, K, r0, ga, gb, vol);
                                 break;
                         }
                     };
@@ -428,6 +438,24 @@ __global__ void volz_kernel(const float* __restrict__ in, int X, int Y, int Zs, 
 }
 
 }  // namespace
+
+int bounds_status_forward(unsigned* count, unsigned long long* first, int reset) {
+#ifdef CTB_BOUNDS_CHECK
+    CTB_CUDA_TRY(cudaMemcpyFromSymbol(count, g_bounds_count, sizeof(unsigned)));
+    CTB_CUDA_TRY(cudaMemcpyFromSymbol(first, g_bounds_first, sizeof(unsigned long long)));
+    if (reset) {
+        const unsigned z = 0;
+        const unsigned long long zz = 0;
+        CTB_CUDA_TRY(cudaMemcpyToSymbol(g_bounds_count, &z, sizeof z));
+        CTB_CUDA_TRY(cudaMemcpyToSymbol(g_bounds_first, &zz, sizeof zz));
+    }
+#else
+    (void)reset;
+    *count = 0;
+    *first = 0;
+#endif
+    return CTB_OK;
+}
 
 int forward_launch(const float* vol, const float4* views, int n_views, const ProjGeom& g, float* proj,
                    int accumulate, cudaStream_t s) {

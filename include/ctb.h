@@ -443,8 +443,8 @@ void ctb_diag_fail_allocation(long nth);
 /* Bounds-checked build (libctb_checked.so, compiled with CTB_BOUNDS_CHECK):
  * the backprojection kernels check every texel fetch against the buffer it
  * reads (the staged box in shared memory, or the projections in global
- * memory), skip a fetch out of range and record it: *violations counts them
- * on `device` since the last reset and *first encodes the first one
+ * memory), the forward projector every voxel against its copy of the slab, skip a
+ * fetch out of range and record it: *violations counts them on `device` since the last reset and *first encodes the first one
  * (site << 56 | index). *checked_build is 0 in the normal library, whose
  * kernels carry no checks (the counts are then 0). reset != 0 clears them.
  * No reference counterpart (compute-sanitizer's memcheck is not used). */
