@@ -65,12 +65,6 @@ inline size_t raw_bytes(int raw_type) { return raw_type == CTB_U8 ? 1 : raw_type
 // threads and a CTA has at most 1024 threads.
 constexpr int kMaxFftLen = 8192;
 
-struct FilterPlan {
-    int W = 0, pad = 0, filter = -1, M = 0, logM = 0;
-    float2* tw = nullptr;   // exp(-2 pi i k / M), k < M, and reordered (FP64-built, stored FP32)
-    float* K = nullptr;     // real kernel spectrum, M entries (includes scaling)
-};
-
 // Transform length for a detector width and padding mode.
 int filter_transform_length(int W, int pad);
 // Build the twiddle and kernel-spectrum tables on the device (FP64 kernels).

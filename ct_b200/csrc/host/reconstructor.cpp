@@ -851,7 +851,8 @@ int Reconstructor::run_pipeline(DeviceWork& w, float* out, int order, int z_lo, 
         (st = w.d_views.ensure(sizeof(float4) * V, "view table")) ||
         (st = w.d_angles.ensure(sizeof(double) * V, "angles")) ||
         (st = w.d_heights.ensure(sizeof(double) * V, "height offsets")) ||
-        (st = w.d_tw.ensure(sizeof(float2) * filter_twiddle_count(M), "twiddles")) || (st = w.d_K.ensure(sizeof(float) * M, "filter")))
+        (st = w.d_tw.ensure(sizeof(float2) * filter_twiddle_count(M), "twiddles")) ||
+        (st = w.d_K.ensure(sizeof(float) * M, "filter")))
         return fail(st, global_error());
     // Slab boundaries: slabs of `slab` slices, and a last one of 32 slices cut
     // from a full-height last slab, so that the download no backprojection

@@ -313,9 +313,9 @@ __global__ void __launch_bounds__(256) repack_rows_kernel(const unsigned char* _
 // and backprojected from there with the shared-memory kernel. The copy reads and
 // writes each sample once; the gather kernel it replaces fetches four samples
 // per voxel and view through L1. 500 views of 1021 x 777 BF16 into 333 x 301
-// x 71: 3.6 ms against 15.2 ms with the gather kernel. The scratch holds 256 MB of views, or as many bytes as the slab if that is
-// more: each run reads and writes the slab once. Returns CTB_ERR_UNSUPPORTED
-// (nothing launched) when it has no memory.
+// x 71: 3.6 ms against 15.2 ms with the gather kernel. The scratch holds 256 MB of
+// views, or as many bytes as the slab if that is more: each run reads and writes the
+// slab once. Returns CTB_ERR_UNSUPPORTED (nothing launched) when it has no memory.
 int backproject_repacked(const void* proj, int store_type, const float4* views, int n_views, const ProjGeom& g,
                          double hmax, float* vol, int accumulate, cudaStream_t s, int zc, int nbuf) {
     const size_t es = store_bytes(store_type);
@@ -396,10 +396,10 @@ int backproject_launch(const void* proj, int store_type, const float4* views, in
         } else if (variant == 0 && cfg.scratch &&
                    (store_type == CTB_FP32 || store_type == CTB_FP16 || store_type == CTB_BF16)) {
             // the copy costs about a fifth (16 bits) to two fifths (32 bits) of a gathered
-            // update per sample: worth it from half an update per copied sample on
-            // (333 x 301 x 71 voxels from 500 views of 1021 x 777 BF16, about 50 updates per
-            // sample: 3.6 ms instead of 15.2; 32^3 voxels from 100 views of 2047 x 1500, 0.2 per sample: gathered
-            // in 0.39 ms, the copy alone moves 60 MB)
+            // update per sample: worth it from half an update per copied sample on (333 x 301 x
+            // 71 voxels from 500 views of 1021 x 777 BF16, about 50 updates per sample: 3.6 ms
+            // instead of 15.2; 32^3 voxels from 100 views of 2047 x 1500, 0.2 per sample:
+            // gathered in 0.39 ms, the copy alone moves 60 MB)
             int lo = 0, rows = 0;
             slab_row_band(g, -hmax, hmax, &lo, &rows);
             const double updates = double(g.X) * g.Y * g.Zs, samples = double(g.W) * rows;

@@ -153,9 +153,6 @@ __device__ __forceinline__ float weight_part(int r, int c, const FilterArgs& a) 
     const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(a.D, a.D), __fmul_rn(u, u)), __fmul_rn(v, v));
     return __fdiv_rn(a.D, __fsqrt_rn(d2));
 }
-__device__ __forceinline__ float preprocess(float s, int r, int c, const FilterArgs& a) {
-    return __fmul_rn(log_part(s, a), weight_part(r, c, a));
-}
 
 // TAB: the Feldkamp weight of every pixel comes from a table (exactly
 // weight_part's values), loaded together with the raw samples, instead of a
@@ -231,13 +228,12 @@ __device__ __forceinline__ void butterfly(float2* v) {
     else dft8<INV>(v);
 }
 
-enum { kFromSmem = 0, kFromInput = 1 };
 enum { kToSmem = 0, kToSmemTimesK = 1, kToOutput = 2 };
 
 // One radix-R stage; each of the TG threads does 8/R butterflies.
-template <int R, bool INV, int SRC, int DST, typename In, typename Out>
+template <int R, bool INV, int DST, typename Out>
 __device__ __forceinline__ void fft_stage(float2* s, int M, int Ns, const float2* __restrict__ tw,
-                                          const float* __restrict__ K, int lt, int TG, const In& in, const Out& out) {
+                                          const float* __restrict__ K, int lt, int TG, const Out& out) {
     constexpr int PER = 8 / R;
     const int nb = M / R;
     const int step = M / (Ns * R);
@@ -247,7 +243,7 @@ __device__ __forceinline__ void fft_stage(float2* s, int M, int Ns, const float2
         const int b = lt + i * TG;
         const int jm = b & (Ns - 1);
 #pragma unroll
-        for (int r = 0; r < R; ++r) y[i][r] = SRC == kFromInput ? in(b + r * nb) : s[b + r * nb];
+        for (int r = 0; r < R; ++r) y[i][r] = s[b + r * nb];
         if (Ns > 1) {
 #pragma unroll
             for (int r = 1; r < R; ++r) {
@@ -258,7 +254,7 @@ __device__ __forceinline__ void fft_stage(float2* s, int M, int Ns, const float2
         }
         butterfly<R, INV>(y[i]);
     }
-    if (SRC == kFromSmem && DST != kToOutput) __syncthreads();  // in place: all reads before any write
+    if (DST != kToOutput) __syncthreads();  // in place: all reads before any write
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
         const int b = lt + i * TG;
@@ -280,27 +276,27 @@ __device__ __forceinline__ void fft_stage(float2* s, int M, int Ns, const float2
     if (DST != kToOutput) __syncthreads();
 }
 
-// Whole transform: first stage from SRC0, last stage to DSTL. All threads of
-// the CTA must call it (barriers).
-template <bool INV, int SRC0, int DSTL, typename In, typename Out>
+// Whole transform from shared memory, last stage to DSTL. All threads of the CTA must
+// call it (barriers).
+template <bool INV, int DSTL, typename Out>
 __device__ void fft_run(float2* s, int M, int logM, const float2* __restrict__ tw, const float* __restrict__ K,
-                        int lt, int TG, const In& in, const Out& out) {
+                        int lt, int TG, const Out& out) {
     const int rem = logM % 3;
     const int first = rem == 1 ? 2 : rem == 2 ? 4 : 8;
     const int nst = logM / 3 + (rem ? 1 : 0);
     int Ns = 1;
     for (int st = 0; st < nst; ++st) {
         if (st == 0) {
-            if (nst == 1) fft_stage<8, INV, SRC0, DSTL>(s, M, Ns, tw, K, lt, TG, in, out);
-            else if (first == 2) fft_stage<2, INV, SRC0, kToSmem>(s, M, Ns, tw, K, lt, TG, in, out);
-            else if (first == 4) fft_stage<4, INV, SRC0, kToSmem>(s, M, Ns, tw, K, lt, TG, in, out);
-            else fft_stage<8, INV, SRC0, kToSmem>(s, M, Ns, tw, K, lt, TG, in, out);
+            if (nst == 1) fft_stage<8, INV, DSTL>(s, M, Ns, tw, K, lt, TG, out);
+            else if (first == 2) fft_stage<2, INV, kToSmem>(s, M, Ns, tw, K, lt, TG, out);
+            else if (first == 4) fft_stage<4, INV, kToSmem>(s, M, Ns, tw, K, lt, TG, out);
+            else fft_stage<8, INV, kToSmem>(s, M, Ns, tw, K, lt, TG, out);
             Ns *= first;
         } else if (st == nst - 1) {
-            fft_stage<8, INV, kFromSmem, DSTL>(s, M, Ns, tw, K, lt, TG, in, out);
+            fft_stage<8, INV, DSTL>(s, M, Ns, tw, K, lt, TG, out);
             Ns *= 8;
         } else {
-            fft_stage<8, INV, kFromSmem, kToSmem>(s, M, Ns, tw, K, lt, TG, in, out);
+            fft_stage<8, INV, kToSmem>(s, M, Ns, tw, K, lt, TG, out);
             Ns *= 8;
         }
     }
@@ -327,23 +323,15 @@ __global__ void __launch_bounds__(1024) filter_kernel(const InT* __restrict__ ra
     const size_t base0 = (size_t)view * H * W + (size_t)r0 * W;              // raw rows (dense)
     const size_t obase = (size_t)view * H * a.out_pitch + (size_t)r0 * a.out_pitch;  // filtered rows
 
-    // rows r0 and r0+1 as the real and imaginary parts, zero beyond W
-    auto load = [&](int c) {
-        float2 z = make_float2(0.f, 0.f);
-        if (active && c < W) {
-            z.x = preprocess(raw_value(raw + base0 + c, a), r0, c, a);
-            if (has1) z.y = preprocess(raw_value(raw + base0 + W + c, a), r0 + 1, c, a);
-        }
-        return z;
-    };
     auto store = [&](int c, float2 z) {
         if (active && c < W) {
             out[obase + c] = to_store<OutT>(z.x * a.store_scale);
             if (has1) out[obase + a.out_pitch + c] = to_store<OutT>(z.y * a.store_scale);
         }
     };
-    // Preprocessing is kept out of the first FFT stage (done there it raises the
-    // register footprint: it involves log, sqrt and divide). All 16 raw loads of
+    // Rows r0 and r0+1 as the real and imaginary parts, zero beyond W. Preprocessing is
+    // kept out of the first FFT stage (done there it raises the register footprint: it
+    // involves log, sqrt and divide). All 16 raw loads of
     // a thread (8 columns x 2 rows; TG = M/8) are issued before any arithmetic,
     // so their latencies overlap instead of adding up.
     InT v0[8], v1[8];
@@ -374,8 +362,8 @@ __global__ void __launch_bounds__(1024) filter_kernel(const InT* __restrict__ ra
         s[c] = z;
     }
     __syncthreads();
-    fft_run<false, kFromSmem, kToSmemTimesK>(s, M, a.logM, tw, K, lt, TG, load, store);
-    fft_run<true, kFromSmem, kToOutput>(s, M, a.logM, tw, K, lt, TG, load, store);
+    fft_run<false, kToSmemTimesK>(s, M, a.logM, tw, K, lt, TG, store);
+    fft_run<true, kToOutput>(s, M, a.logM, tw, K, lt, TG, store);
 }
 
 // --------------------------------------- register four-step transform
@@ -542,9 +530,11 @@ __device__ __forceinline__ C2 as2(const float4& a) { return {make_float2(a.x, a.
 
 // -ln of two positive normal numbers. With m in [sqrt(1/2), sqrt(2)) the number's
 // mantissa, e its exponent and n = 1 - m (exact): -ln m = n + n^2 Q(n), Q a degree-8
-// least-maximum-error fit of the relative error over the interval (4e-9), and e ln 2
-// is taken off in two parts, the first exact for every e. Within about one unit in
-// the last place, as logf; the FP32x2 form shares each step between two samples.
+// least-maximum-error fit of the relative error over the interval (its coefficients
+// rounded to floats leave 7e-9), and e ln 2 is taken off in two parts, the first
+// exact for every e: Cody and Waite's reduction (Software Manual for the Elementary
+// Functions, 1980) with the mantissa about 1. At most 0.9 units in the last place
+// of the result, as logf; the FP32x2 form shares each step between two samples.
 __device__ __forceinline__ float2 neg_ln2(float2 s) {
     const int ix = __float_as_int(s.x) - 0x3F3504F3, iy = __float_as_int(s.y) - 0x3F3504F3;   // bits of sqrt(1/2)
     const int ex = ix & 0xff800000, ey = iy & 0xff800000;                                     // e << 23

@@ -26,8 +26,9 @@
 //     becomes a record in shared memory;
 //  3. the warp takes the step's records, those with the same u0 and window
 //     length together. For its row r a lane sums the column's slices z with
-//     their vertical weights 1 - |vi(z) - r| (the bilinear weights 1-fv and fv
-//     of rows v0 and v0+1, exactly: the differences are exact in FP32); only
+//     their vertical weights 1 - |vi(z) - r|, the bilinear weights 1-fv and fv
+//     of rows v0 and v0+1 (exactly, the differences being exact in FP32 but for
+//     vi - 1 below row 1/2, which rounds by less than 2^-24); only
 //     the K = floor(2 / dv) + 1 slices from (c0 - r - 1) / dv on can have one,
 //     dv the rows per slice. The sum times w (1-fu) and w fu goes to columns
 //     u0 and u0+1: two registers per row within a group of records, the
@@ -361,8 +362,8 @@ __global__ void __launch_bounds__(32 * kWarps, 7) fp_kernel(const float* __restr
                         const Hit t = sh.hits[src];
 #pragma unroll
                         for (int j = 0; j < J; ++j) {
-                            const float x = checked_sum(t.line + kMagicBits, fmaf(-(r0 + 32.0f * j), t.inv, t.za), K, a, b,
-                                                        t.mdv, t.c0, R + lane + 32 * j, vol);
+                            const float x = checked_sum(t.line + kMagicBits, fmaf(-(r0 + 32.0f * j), t.inv, t.za), K, a,
+                                                        b, t.mdv, t.c0, R + lane + 32 * j, vol);
                             float& xa = j & 1 ? ga[j / 2].y : ga[j / 2].x;
                             float& xb = j & 1 ? gb[j / 2].y : gb[j / 2].x;
                             xa = fmaf(t.wa, x, xa);
