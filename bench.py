@@ -295,6 +295,13 @@ def scan_seed(rank: int) -> int:
     return 1000 + rank
 
 
+def columns_inside(det, grid) -> float:
+    """Share of the box's voxel columns that lie inside the reconstruction cylinder."""
+    x = (np.arange(grid.x_from, grid.x_to) - grid.x_size / 2.0) * grid.voxel_pitch
+    y = (np.arange(grid.y_from, grid.y_to) - grid.y_size / 2.0) * grid.voxel_pitch
+    return float((x[None, :] ** 2 + y[:, None] ** 2 < det.radius ** 2).mean())
+
+
 def whole_job_gups(voxel_views_per_rank: float, world: int, ms_per_step: float) -> float:
     """Whole-job throughput: the units all ranks processed over the max-over-ranks step time."""
     return voxel_views_per_rank * world / (ms_per_step * 1e-3) / 1e9
@@ -786,16 +793,18 @@ def run_ours(args):
     sm_count = torch.cuda.get_device_properties(local).multi_processor_count
     # fetch roofline: one bilinear sample = 4 texel loads; the L1/shared load path serves one
     # warp-wide (32-lane) load instruction per SM per clock
+    # over the updates made: columns outside the reconstruction cylinder fetch nothing
     peak_gups = sm_count * clock_mhz * 1e6 * 32 / 4 / 1e9
-    bp_gups = units / (main["bp_ms"] * 1e-3) / 1e9
+    made = columns_inside(det, grid)
+    bp_gups = made * units / (main["bp_ms"] * 1e-3) / 1e9
     bytes_px_in, bytes_px_out = 2, (2 if store != L.FP32 else 4)
     filt_gbs = V * H * W * (bytes_px_in + bytes_px_out) / (main["filter_ms"] * 1e-3) / 1e9
     roofline = {"bound": "fetch", "kernel": "bp_tma_kernel", "achieved": bp_gups, "peak": peak_gups, "unit": "GUPS",
-                "frac": bp_gups / peak_gups,
+                "frac": bp_gups / peak_gups, "updates_made_of_voxel_views": made,
                 "traffic": (BP_DRAM_BYTES_PER_UPDATE[(args.config, slab)] * X * Y * slab * V
                             if (args.config, slab) in BP_DRAM_BYTES_PER_UPDATE and args.store == "fp16" else None),
                 "traffic_unit": "DRAM bytes per backprojection launch (one slab)",
-                "algorithmic_bytes_per_launch": 8.0 * X * Y * slab * V,
+                "algorithmic_bytes_per_launch": 8.0 * made * X * Y * slab * V,
                 "peak_basis": f"{sm_count} SMs x {clock_mhz:.0f} MHz (median sampled) x 32 lanes / 4 texel loads"}
     fft_len = W if W & (W - 1) == 0 else 1 << (2 * W - 2).bit_length()   # transform length of the row filter
     filt_kernel = "filter_rf_kernel" if 512 <= fft_len <= 4096 else "filter_kernel"
